@@ -93,7 +93,7 @@ def listed():
         # The moving image carried onto the fixed grid at a registration's
         # end.
         _case("warp", (256, 256, 128), (0.98, 0.98, 2.5), (5, 5, 5),
-              "warp_256x256x128_vpr5"),
+              "warp_256x256x128_vpr5", pad=MARGIN),
     ]
 
 
@@ -123,7 +123,9 @@ def draw(rng):
     if kind == "mi":
         kw = {"window": rng.choice(["pvi8", "parzen"]), "bins": rng.choice([20, 32, 48])}
         pad = MARGIN
-    elif kind != "warp":
+    elif kind == "warp":
+        pad = MARGIN
+    else:
         kw["grad"] = rng.choice(["nearest", "nearest", "trilinear"])
         if kind == "mse":
             pad = tuple(rng.randint(-6, 10) for _ in range(3))
