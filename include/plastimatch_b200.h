@@ -41,7 +41,8 @@ extern "C" {
 #define B200BSP_E_IO           -7   /* file missing, unreadable or malformed */
 
 /* Kernel forms. */
-#define B200BSP_FORM_TC    0   /* tcgen05 tensor-core field + adjoint (default) */
+#define B200BSP_FORM_TC    0   /* the fast kernels (default): the line kernel, or
+                                  tcgen05 tensor-core field + adjoint */
 #define B200BSP_FORM_FP32  1   /* plain FP32 SIMT, one thread per voxel */
 
 /* MSE gradient semantics. */
@@ -83,16 +84,20 @@ typedef struct {
     int tc_kernel;      /* B200BSP_TC_KERNEL_* (0: chosen per context) */
 } b200bsp_opts;
 
-/* The tensor-core form's MSE kernel.  AUTO starts on the tile kernel (the
- * voxels of one tile on the TMEM lanes); b200bsp_autotune may move it to
- * the x-lane kernel (voxel x on the lanes, 3 <= vox_per_rgn[1] <= 10) and
- * back, and image ROIs (b200bsp_set_roi) move it to the x-lane kernel,
- * which is the one that tests them.  XLANE and TILE pin one (XLANE on a
- * grid it cannot take is B200BSP_E_UNSUPPORTED; with TILE pinned, image
- * ROIs are B200BSP_E_UNSUPPORTED in the tensor-core form). */
+/* The tensor-core form's MSE kernel.  AUTO runs the line kernel (FP32,
+ * separable, marching along y) on grids with 3 to 10 voxels a region on
+ * every axis, with or without image ROIs.  On other grids it starts on the
+ * tile kernel (the voxels of one tile on the TMEM lanes); b200bsp_autotune
+ * may move it to the x-lane kernel (voxel x on the lanes, 3 <=
+ * vox_per_rgn[1] <= 10) and back, and image ROIs (b200bsp_set_roi) move it
+ * to the x-lane kernel.  XLANE and TILE pin one of the tensor-core kernels
+ * (XLANE on a grid it cannot take is B200BSP_E_UNSUPPORTED; with TILE
+ * pinned, image ROIs are B200BSP_E_UNSUPPORTED in the tensor-core form). */
 #define B200BSP_TC_KERNEL_AUTO   0
 #define B200BSP_TC_KERNEL_XLANE  1
 #define B200BSP_TC_KERNEL_TILE   2
+/* b200bsp_mse_kernel's name for the line kernel. */
+#define B200BSP_MSE_KERNEL_LINE  3
 
 /* Mattes MI histogram windows: PVI-8 partial-volume binning (the
  * reference's, bspline_mi.cxx) or cubic B-spline Parzen windows on the
@@ -299,14 +304,16 @@ int b200bsp_mi_grad (b200bsp_ctx* ctx, const float* coeff,
  * into batches (the fewest batches of at most 26 tiles, and up to two
  * more) and keeps the fastest for the context's later calls; *tiles
  * receives its tiles per batch (1 for the FP32 form, which has nothing to
- * tune).  Results stay within the parity bars whatever the split, and are
+ * tune; the tiles one warp meets along x for the line kernel, whose plan
+ * follows from the grid).  Results stay within the parity bars whatever the split, and are
  * deterministic for a given split. */
 int b200bsp_autotune (b200bsp_ctx* ctx, const float* coeff, int evals,
     int* tiles);
 
 /* The MSE kernel the context's next evaluation runs: *kernel receives
- * B200BSP_TC_KERNEL_XLANE or _TILE (AUTO never; 0 for the FP32 form),
- * *tiles its tiles per batch and *batches the batches it launches. */
+ * B200BSP_TC_KERNEL_XLANE or _TILE (AUTO never), B200BSP_MSE_KERNEL_LINE,
+ * or 0 for the FP32 form; *tiles its tiles per batch (line kernel: tiles a
+ * warp meets along x) and *batches the batches (blocks) it launches. */
 int b200bsp_mse_kernel (const b200bsp_ctx* ctx, int* kernel, int* tiles,
     int* batches);
 

@@ -451,12 +451,12 @@ class Context:
         return t.value
 
     def mse_kernel(self):
-        """b200bsp_mse_kernel: ("xlane" | "tile" | "fp32", tiles per
-        batch, batches) of the next MSE evaluation."""
+        """b200bsp_mse_kernel: ("line" | "xlane" | "tile" | "fp32", tiles
+        per batch, batches) of the next MSE evaluation."""
         k, t, b = C.c_int(), C.c_int(), C.c_int()
         _check(lib().b200bsp_mse_kernel(self._h, C.byref(k), C.byref(t),
                                         C.byref(b)), self._h)
-        name = {0: "fp32", 1: "xlane", 2: "tile"}[k.value]
+        name = {0: "fp32", 1: "xlane", 2: "tile", 3: "line"}[k.value]
         return name, t.value, b.value
 
     def score_mse_f64(self, coeff):

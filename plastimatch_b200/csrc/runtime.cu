@@ -22,6 +22,7 @@
 
 #include "../../include/plastimatch_b200.h"
 #include "kernels.cuh"
+#include "line.cuh"
 #include "mi.cuh"
 #include "regularize.cuh"
 
@@ -75,6 +76,11 @@ struct b200bsp_ctx {
     void* d_xtab = nullptr;
     unsigned wait_limit = XL_DEFAULT_WAIT_LIMIT;
     int withhold_mma = 0;     // b200bsp_set_wait_limit's testing aid
+    // the line kernel (line.cu), an AUTO context's choice on the grids that
+    // line_plan takes
+    bool use_line = false;
+    LinePlan lplan;
+    float* d_rows = nullptr;
     // b200bsp_score's device path: the regulariser on a second stream,
     // overlapping the tile kernel, its gradient kept in double
     double* d_reg_grad64 = nullptr;
@@ -288,6 +294,7 @@ free_all (b200bsp_ctx* c)
     cudaFree (c->d_fixed); cudaFree (c->d_moving); cudaFree (c->d_mgrad);
     cudaFree (c->d_out);
     cudaFree (c->d_mgrad4);
+    cudaFree (c->d_rows);
     if (c->ev_fork) cudaEventDestroy (c->ev_fork);
     if (c->ev_join) cudaEventDestroy (c->ev_join);
     if (c->aux_stream) cudaStreamDestroy (c->aux_stream);
@@ -643,6 +650,13 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
                 }
                 use_xl_plan (c, c->xplan);
             }
+            if (o.tc_kernel == B200BSP_TC_KERNEL_AUTO
+                && line_plan (g, &c->lplan, sm_count)) {
+                c->use_line = true;
+                alloc ((void**) &c->d_rows, line_row_elems (g, c->lplan)
+                    * sizeof (float));
+                score_parts = std::max (score_parts, (size_t) c->lplan.nblocks);
+            }
         }
     } else if (!rc2) {
         if (mse_fp32_smem_bytes (g) > 200 * 1024) {
@@ -717,6 +731,9 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
         cudaMemcpyHostToDevice);
     cudaMemcpy (c->d_inv_dc, minv, 9 * sizeof (float), cudaMemcpyHostToDevice);
     cudaMemset (c->d_err, 0, sizeof (int));
+    if (c->use_line) {
+        cudaMemset (c->d_rows, 0, line_row_elems (g, c->lplan) * sizeof (float));
+    }
     if (cudaDeviceSynchronize () != cudaSuccess) {
         std::string e = cudaGetErrorString (cudaGetLastError ());
         free_all (c);
@@ -732,7 +749,8 @@ b200bsp_set_wait_limit (b200bsp_ctx* c, int polls, int withhold_mma)
 {
     if (!c) return B200BSP_E_BADARG;
     if (polls < 0) return fail (c, B200BSP_E_BADARG, "polls must be >= 0");
-    if (withhold_mma && !(c->opts.form == B200BSP_FORM_TC && c->use_xl)) {
+    if (withhold_mma && !(c->opts.form == B200BSP_FORM_TC && c->use_xl
+            && !c->use_line)) {
         return fail (c, B200BSP_E_UNSUPPORTED,
             "withholding MMAs is a testing aid of the x-lane kernel");
     }
@@ -895,6 +913,10 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
         CK (launch_mse_fp32 (g, c->opts.mse_grad, c->d_fixed, c->d_moving,
             c->d_mgrad, dcoeff, c->d_luts, c->d_part, c->d_score_part,
             c->d_count_part, c->stream));
+    } else if (c->use_line) {
+        CK (launch_mse_line (g, c->lplan, c->opts.mse_grad, c->d_fixed,
+            c->d_moving, c->d_mgrad4, dcoeff, c->d_luts, c->d_rows,
+            c->d_score_part, c->d_count_part, c->stream));
     } else if (c->use_xl) {
         XlPlan plan = c->xplan;
         // a batch's share of the SMs' CTA slots counts two per SM (the
@@ -923,6 +945,14 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
     }
     const bool xl = c->opts.form == B200BSP_FORM_TC && c->use_xl;
     if (before_finish) CK (cudaStreamWaitEvent (c->stream, before_finish, 0));
+    if (c->use_line) {
+        CK (launch_line_finish (g, c->lplan, c->d_rows, c->d_luts,
+            c->d_score_part, c->d_count_part, c->lplan.nblocks, c->d_err,
+            c->d_res, res_host, grad_out, grad64_out, score_out, score64_out,
+            nvox_out, c->stream, combine));
+        c->last_launches += 1;
+        return B200BSP_OK;
+    }
     CK (launch_finish_mse (g, xl ? c->xlay : c->lay, c->d_part,
         c->d_score_part, c->d_count_part,
         xl ? c->xplan.score_parts : c->nscore_parts,
@@ -1028,6 +1058,11 @@ b200bsp_autotune (b200bsp_ctx* c, const float* coeff, int evals, int* tiles)
     const float* dcoeff = nullptr;
     int rc = begin_eval (c, coeff, &dcoeff);
     if (rc) return rc;
+    if (c->use_line) {
+        // its plan follows from the grid: nothing to choose
+        if (tiles) *tiles = c->lplan.kx;
+        return B200BSP_OK;
+    }
     int sm_count = 148;
     cudaDeviceGetAttribute (&sm_count, cudaDevAttrMultiProcessorCount,
         c->device);
@@ -1107,7 +1142,11 @@ b200bsp_mse_kernel (const b200bsp_ctx* c, int* kernel, int* tiles,
 {
     if (!c) return B200BSP_E_BADARG;
     int k = 0, t = 1, b = c->geom.ntiles;
-    if (c->opts.form == B200BSP_FORM_TC && c->use_xl) {
+    if (c->use_line) {
+        k = B200BSP_MSE_KERNEL_LINE;
+        t = c->lplan.kx;
+        b = c->lplan.nblocks;
+    } else if (c->opts.form == B200BSP_FORM_TC && c->use_xl) {
         k = B200BSP_TC_KERNEL_XLANE;
         t = c->xplan.T;
         b = c->xplan.nbatches;

@@ -1,0 +1,80 @@
+"""The line kernel (what a tensor-core-form context runs by default on grids
+with 3 to 10 voxels a region) against the FP32 form's tile kernel, at the
+edges of its blocks: warps and blocks partly beyond the ROI, ragged last
+tiles, the smallest and largest regions, rotated axes, partial ROIs, images
+wider than one finish block.
+
+Both kernels work in float and differ in the order of their sums: the field
+by a few units of 2^-24 of the coefficients, the gradient by the rounding of
+sums of at most 4 x 4 x 4 tiles of 1000 voxels (grouped, < 100 roundings
+deep), i.e. 100 x 2^-24 = 6e-6; a voxel whose position falls on the other
+side of a cell's face changes its own term only (images without noise: the
+moving gradient is smooth).  Bars: score 2e-6, gradient 2e-5, count 1e-4 + 2.
+"""
+import numpy as np
+import pytest
+
+import plastimatch_b200 as P
+from conftest import rel_err
+from plastimatch_b200 import synth
+from plastimatch_b200.geometry import BsplineGrid, Volume
+
+pytestmark = pytest.mark.gpu
+
+# dims, vox_per_rgn, ROI (offset, dim) or None, rotation about z (degrees)
+CASES = [
+    ((24, 24, 24), (4, 4, 4), None, 0.0),
+    ((33, 9, 7), (3, 3, 3), None, 0.0),            # one lane in the last warp
+    ((65, 41, 30), (10, 3, 9), None, 8.0),
+    ((129, 31, 17), (5, 10, 10), None, 0.0),       # two planes in the last row
+    ((64, 64, 64), (3, 10, 10), None, 5.0),
+    ((31, 200, 11), (7, 4, 3), None, 0.0),         # less than a warp along x
+    ((70, 50, 40), (6, 5, 7), ((5, 3, 2), (57, 41, 31)), 0.0),
+    ((1040, 20, 12), (10, 6, 4), None, 0.0),       # two finish blocks along x
+    ((48, 44, 36), (8, 9, 6), ((1, 0, 3), (47, 44, 33)), -15.0),
+]
+
+
+def _volume(dim, seed, dcos, origin=(0.0, 0.0, 0.0)):
+    v = synth.gaussian_blobs(dim, spacing=(1.0, 1.1, 1.6), seed=seed,
+                             noise_sigma=0.0)
+    return Volume(v.img, origin=origin, spacing=v.spacing, dcos=dcos)
+
+
+def _case(dim, vpr, roi, angle, seed=71):
+    a = np.deg2rad(angle)
+    dcos = (np.cos(a), -np.sin(a), 0.0, np.sin(a), np.cos(a), 0.0, 0.0, 0.0, 1.0)
+    fixed = _volume(dim, seed, dcos)
+    # another extent and place: some voxels land outside on every axis
+    moving = _volume((dim[0] - 2, dim[1] + 3, dim[2] + 1), seed, dcos,
+                     (0.4, -0.7, 0.3))
+    kw = dict(roi_offset=roi[0], roi_dim=roi[1]) if roi else {}
+    grid = BsplineGrid.for_volume(fixed, vpr, **kw)
+    return fixed, moving, grid, synth.random_coeff(grid, 1.5, seed + 2)
+
+
+@pytest.mark.parametrize("grad", ["nearest", "trilinear"])
+@pytest.mark.parametrize("case", CASES)
+def test_line_kernel_matches_tile_kernel(case, grad):
+    fixed, moving, grid, coeff = _case(*case)
+    out = []
+    for form in ("fp32", "tc"):
+        with P.Context(fixed, moving, grid, form=form, mse_grad=grad) as ctx:
+            ctx.set_images()
+            name = ctx.mse_kernel()[0]
+            assert name == ("fp32" if form == "fp32" else "line")
+            out.append(ctx.score_mse(coeff))
+            again = ctx.score_mse(coeff)
+            assert again[0] == out[-1][0] and again[2] == out[-1][2]
+            np.testing.assert_array_equal(again[1], out[-1][1])
+    (s0, g0, n0), (s1, g1, n1) = out
+    assert n0 > 0 and abs(n1 - n0) <= 1e-4 * n0 + 2, (n1, n0)
+    assert abs(s1 - s0) <= 2e-6 * abs(s0), (s1, s0)
+    assert rel_err(g1, g0) < 2e-5, rel_err(g1, g0)
+
+
+def test_regions_outside_the_line_kernel_keep_the_tile_kernel():
+    f = _volume((40, 48, 24), 3, (1, 0, 0, 0, 1, 0, 0, 0, 1))
+    for vpr in ((5, 12, 5), (2, 5, 5), (5, 5, 11)):
+        with P.Context(f, f, BsplineGrid.for_volume(f, vpr)) as ctx:
+            assert ctx.mse_kernel()[0] == "tile"
