@@ -86,7 +86,9 @@ typedef struct {
 
 /* The tensor-core form's MSE kernel.  AUTO runs the line kernel (FP32,
  * separable, marching along y) on grids with 3 to 10 voxels a region on
- * every axis, with or without image ROIs.  On other grids it starts on the
+ * every axis, with or without image ROIs, for every evaluation but the
+ * optimiser's (which amplifies the last bits of a gradient and keeps to the
+ * tensor-core kernels).  There, and on other grids, it starts on the
  * tile kernel (the voxels of one tile on the TMEM lanes); b200bsp_autotune
  * may move it to the x-lane kernel (voxel x on the lanes, 3 <=
  * vox_per_rgn[1] <= 10) and back, and image ROIs (b200bsp_set_roi) move it
@@ -304,8 +306,8 @@ int b200bsp_mi_grad (b200bsp_ctx* ctx, const float* coeff,
  * into batches (the fewest batches of at most 26 tiles, and up to two
  * more) and keeps the fastest for the context's later calls; *tiles
  * receives its tiles per batch (1 for the FP32 form, which has nothing to
- * tune; the tiles one warp meets along x for the line kernel, whose plan
- * follows from the grid).  Results stay within the parity bars whatever the split, and are
+ * tune).  The line kernel's plan follows from the grid; on its contexts the
+ * choice is that of the optimiser's evaluations.  Results stay within the parity bars whatever the split, and are
  * deterministic for a given split. */
 int b200bsp_autotune (b200bsp_ctx* ctx, const float* coeff, int evals,
     int* tiles);

@@ -39,7 +39,32 @@
 
 namespace b200 {
 
-enum LineMode { LN_MSE_NEAREST, LN_MSE_LINEAR };
+// What a block does at each voxel: MSE with the nearest or the trilinear
+// moving gradient; Mattes MI pass 1 (PVI-8 or Parzen histograms) and, for
+// Parzen windows, pass 2 (dc/dv from the factor table); the field itself;
+// the warped moving image.
+enum LineMode {
+    LN_MSE_NEAREST, LN_MSE_LINEAR, LN_MI_HIST, LN_PZ_HIST, LN_PZ_GRAD,
+    LN_FIELD, LN_WARP
+};
+
+constexpr bool
+ln_mse (int mode)
+{
+    return mode == LN_MSE_NEAREST || mode == LN_MSE_LINEAR;
+}
+
+constexpr bool
+ln_hist (int mode)
+{
+    return mode == LN_MI_HIST || mode == LN_PZ_HIST;
+}
+
+constexpr bool
+ln_adjoint (int mode)
+{
+    return ln_mse (mode) || mode == LN_PZ_GRAD;
+}
 
 constexpr int LN_MAX_WARPS = 16;
 constexpr int LN_REGS = 64;             // four blocks of eight warps per SM
@@ -58,6 +83,15 @@ struct LineArgs {
     float* rows;         // adjoint rows [z][y block][j][c][nxs]
     double* score_part;
     int* count_part;
+    const uint8_t* fbin; // MI: fixed bin per voxel
+    const uint32_t* mquad;                  // PVI-8: bins of 2 x 2 moving voxels
+    const float* lut;    // Parzen pass 2: [fixed bin][moving bin] factors
+    const float* nvf;    //   [1]: 1 / (N delta_m)
+    u64* hist;           // pass 1: f[B], m[B], j[B * B], count
+    int bins;
+    float pz_min, pz_inv;                   // moving value -> window centre
+    float* out;          // field (xyz per voxel) or warped image
+    float outside;
     int ty, j, nxs;
     u64 step_y;          // AXIS: (0, fixed y step)
     u64 morg, mprj;      // AXIS: moving x and y origin and projection
@@ -156,6 +190,8 @@ struct Vox {
     float cr[8], fv;
     float4 gr;
     float w2[3];
+    uint32_t mq[2];
+    int fb, fidx, clamp;
     bool ok;
 };
 
@@ -227,6 +263,7 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
     jf2 = add2 (jf2, pk (1.f, 1.f));
     bool in = col.live;
     int bits[3];
+    v.clamp = 0;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         in = in && ma[d] > -0.5f && ma[d] < g.m_hi[d];
@@ -236,10 +273,20 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
         bits[d] = min (__float_as_int (__fadd_rd (fmaxf (ma[d], 0.f),
             8388608.f)), a.mtop[d]);
         v.w2[d] = __saturatef (ma[d] - (__int_as_float (bits[d]) - 8388608.f));
+        if (MODE == LN_PZ_GRAD && (ma[d] < 0.f || ma[d] >= g.m_fmax[d] + 1.f)) {
+            v.clamp |= 1 << d;
+        }
     }
     const int mvf = bits[0] + g.mdim[0] * (bits[1] + g.mdim[1] * bits[2])
         + a.midx0;
     const int fidx = col.frow + fj * g.fdim[0];
+    v.fidx = fidx;
+    if (MODE == LN_FIELD) {
+        v.cr[0] = lo2 (dxy);
+        v.cr[1] = hi2 (dxy);
+        v.cr[2] = dz;
+        return;
+    }
     if (ROI) {
         const float dd[3] = {lo2 (dxy), hi2 (dxy), dz};
         in = in && roi_fixed_ok (g, fidx);
@@ -257,7 +304,13 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
             + (v.w2[1] >= 0.5f ? dx : 0) + (v.w2[2] >= 0.5f ? dxym : 0);
         v.gr = ld4 (a.mgrad4 + mvr);
     }
-    v.fv = ld1 (a.fimg + fidx);
+    if (ln_mse (MODE)) v.fv = ld1 (a.fimg + fidx);
+    if (ln_hist (MODE) || MODE == LN_PZ_GRAD) v.fb = __ldg (a.fbin + fidx);
+    if (MODE == LN_MI_HIST) {
+        v.mq[0] = __ldg (a.mquad + mvf);
+        v.mq[1] = __ldg (a.mquad + mvf + dxym);
+        return;
+    }
     v.cr[0] = ld1 ((const float*) (b0 + off));
     v.cr[1] = ld1 ((const float*) (b0 + off) + 1);
     v.cr[2] = ld1 ((const float*) (b1 + off));
@@ -268,20 +321,44 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
     v.cr[7] = ld1 ((const float*) (b3 + off) + 1);
 }
 
-// The metric at a loaded voxel and its adjoint.
-template <int MODE, int R>
-__device__ __forceinline__ void
-line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
-    Row (&q)[4], float& scf, int& cnt)
+// Trilinear value (x, then y, then z; the z planes' lerps in pairs, with the
+// rounding of trilinear_lerp).
+__device__ __forceinline__ float
+line_value (const Vox& v)
 {
-    // the z planes' lerps along x and y in pairs (same rounding)
     const u64 wx2 = pk (v.w2[0], v.w2[0]), wy2 = pk (v.w2[1], v.w2[1]);
     const u64 m0 = pk (v.cr[0], v.cr[4]), m1 = pk (v.cr[1], v.cr[5]);
     const u64 m2 = pk (v.cr[2], v.cr[6]), m3 = pk (v.cr[3], v.cr[7]);
     const u64 c0 = fma2 (wx2, sub2 (m1, m0), m0);
     const u64 c1 = fma2 (wx2, sub2 (m3, m2), m2);
     const u64 cc = fma2 (wy2, sub2 (c1, c0), c0);
-    float diff = fmaf (v.w2[2], hi2 (cc) - lo2 (cc), lo2 (cc)) - v.fv;
+    return fmaf (v.w2[2], hi2 (cc) - lo2 (cc), lo2 (cc));
+}
+
+// dc/dv of one voxel (y weights wy) into the window of adjoint rows.
+template <int R>
+__device__ __forceinline__ void
+line_adjoint (const ulonglong2* __restrict__ wy, u64 cxy, float cz,
+    Row (&q)[4])
+{
+    const ulonglong2 w01 = wy[0], w23 = wy[1];
+    q[R].xy = fma2 (w01.x, cxy, q[R].xy);
+    q[R].z = fmaf (lo2 (w01.x), cz, q[R].z);
+    q[(R + 1) & 3].xy = fma2 (w01.y, cxy, q[(R + 1) & 3].xy);
+    q[(R + 1) & 3].z = fmaf (lo2 (w01.y), cz, q[(R + 1) & 3].z);
+    q[(R + 2) & 3].xy = fma2 (w23.x, cxy, q[(R + 2) & 3].xy);
+    q[(R + 2) & 3].z = fmaf (lo2 (w23.x), cz, q[(R + 2) & 3].z);
+    q[(R + 3) & 3].xy = fma2 (w23.y, cxy, q[(R + 3) & 3].xy);
+    q[(R + 3) & 3].z = fmaf (lo2 (w23.y), cz, q[(R + 3) & 3].z);
+}
+
+// MSE at a loaded voxel and its adjoint.
+template <int MODE, int R>
+__device__ __forceinline__ void
+line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
+    Row (&q)[4], float& scf, int& cnt)
+{
+    float diff = line_value (v) - v.fv;
     diff = v.ok ? diff : 0.f;
     scf = fmaf (diff, diff, scf);
     cnt += v.ok ? 1 : 0;
@@ -296,15 +373,168 @@ line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
         cxy = mul2 (pk (diff, diff), pk (gd[0], gd[1]));
         cz = diff * gd[2];
     }
-    const ulonglong2 w01 = wy[0], w23 = wy[1];
-    q[R].xy = fma2 (w01.x, cxy, q[R].xy);
-    q[R].z = fmaf (lo2 (w01.x), cz, q[R].z);
-    q[(R + 1) & 3].xy = fma2 (w01.y, cxy, q[(R + 1) & 3].xy);
-    q[(R + 1) & 3].z = fmaf (lo2 (w01.y), cz, q[(R + 1) & 3].z);
-    q[(R + 2) & 3].xy = fma2 (w23.x, cxy, q[(R + 2) & 3].xy);
-    q[(R + 2) & 3].z = fmaf (lo2 (w23.x), cz, q[(R + 2) & 3].z);
-    q[(R + 3) & 3].xy = fma2 (w23.y, cxy, q[(R + 3) & 3].xy);
-    q[(R + 3) & 3].z = fmaf (lo2 (w23.y), cz, q[(R + 3) & 3].z);
+    line_adjoint<R> (wy, cxy, cz, q);
+}
+
+// Parzen pass 2 at a loaded voxel: 1/(N delta_m) * sum over the window's
+// bins of beta3'(k - u) log(p(f, k) / p_m(k)) (slut, shared memory), times
+// the world gradient of the trilinear interpolant (proj^T times the index
+// gradient; 0 along an axis the clamp holds).  With f = u - floor(u) the
+// window's derivative at its four bins is (1-f)^2/2, 2f - 3f^2/2,
+// -2s + 3s^2/2 (s = 1-f) and -f^2/2.
+template <bool AXIS, int R>
+__device__ __forceinline__ void
+line_use_pz (const LineArgs& a, const ulonglong2* __restrict__ wy,
+    const Vox& v, const float* slut, float scale, Row (&q)[4])
+{
+    const float u = fmaf (line_value (v) - a.pz_min, a.pz_inv, 2.f);
+    const int k0 = parzen_first_bin (u, a.bins);
+    const float f = u - (float) (k0 + 1), s = 1.f - f;
+    const float* row = slut + v.fb * a.bins + k0;
+    const float sum = (0.5f * s * s) * row[0] + (f * fmaf (-1.5f, f, 2.f)) * row[1]
+        + (s * fmaf (1.5f, s, -2.f)) * row[2] - (0.5f * f * f) * row[3];
+    float gi[3];
+    trilinear_igrad (v.w2, v.cr, v.clamp, gi);
+    const float sc = v.ok ? scale * sum : 0.f;
+    const float* p = a.g.mproj;
+    float dc[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        dc[c] = AXIS ? sc * (p[4 * c] * gi[c])
+                     : sc * (p[c] * gi[0] + p[3 + c] * gi[1] + p[6 + c] * gi[2]);
+    }
+    line_adjoint<R> (wy, pk (dc[0], dc[1]), dc[2], q);
+}
+
+// Histograms of a block: weights are summed as integers in 2^-24 units (no
+// float atomics, any order).  A thread keeps the sums of the bin (pair) its
+// last voxels fell into and adds them to shared memory only when the next
+// voxel falls into another, as two 16-bit halves in 32-bit counters: shared
+// 32-bit adds are native, and a block of fewer than 65536 voxels cannot
+// overflow them (line_plan: one sum a voxel and bin).
+struct Run {
+    int key;             // joint bin (Parzen: the first of four); -1: none
+    uint32_t s[4];       // weights (PVI-8: [0] the weight, [1] the voxels)
+};
+
+__device__ __forceinline__ void
+hist_add (uint32_t* sh, int nj, int bin, uint32_t w)
+{
+    atomicAdd (sh + bin, w & 0xffffu);
+    atomicAdd (sh + nj + bin, w >> 16);
+}
+
+template <int MODE>
+__device__ __forceinline__ void
+hist_flush (uint32_t* sh, int B, const Run& r)
+{
+    const int nj = B * B;
+    if (MODE == LN_PZ_HIST) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) hist_add (sh, nj, r.key + j, r.s[j]);
+    } else {
+        hist_add (sh, nj, r.key, r.s[0]);
+        atomicAdd (sh + 2 * nj + r.key / B, r.s[1]);
+    }
+}
+
+// Parzen pass 1 at a loaded voxel: the cubic window's four weights at the
+// moving value into the fixed bin's row.
+__device__ __forceinline__ void
+line_use_pz_hist (const LineArgs& a, const Vox& v, uint32_t* sh, Run& r)
+{
+    if (!v.ok) return;
+    const float u = fmaf (line_value (v) - a.pz_min, a.pz_inv, 2.f);
+    const int k0 = parzen_first_bin (u, a.bins);
+    const float f = u - (float) (k0 + 1), s = 1.f - f;
+    const float f2 = f * f, s2 = s * s;
+    const float w0 = s2 * s * (1.f / 6.f), w3 = f2 * f * (1.f / 6.f);
+    const float w1 = fmaf (f2, fmaf (0.5f, f, -1.f), 2.f / 3.f);
+    const float w2 = fmaf (s2, fmaf (0.5f, s, -1.f), 2.f / 3.f);
+    const uint32_t q[4] = {__float2uint_rn (w0 * 16777216.f),
+        __float2uint_rn (w1 * 16777216.f), __float2uint_rn (w2 * 16777216.f),
+        __float2uint_rn (w3 * 16777216.f)};
+    const int key = v.fb * a.bins + k0;
+    if (key != r.key) {
+        if (r.key >= 0) hist_flush<LN_PZ_HIST> (sh, a.bins, r);
+        r.key = key;
+#pragma unroll
+        for (int j = 0; j < 4; j++) r.s[j] = q[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) r.s[j] += q[j];
+    }
+}
+
+// PVI-8 pass 1 at a loaded voxel: the eight corner weights into the joint
+// bins of (fixed bin, corner's bin).  The first corner's bin takes part in
+// the thread's run, with the voxel's count; corners in other bins (edges of
+// structures) go straight to shared memory, those of the first such bin
+// together.  Where all eight share one bin their weights add up to one.
+__device__ __forceinline__ void
+line_use_mi_hist (const LineArgs& a, const Vox& v, uint32_t* sh, Run& r)
+{
+    if (!v.ok) return;
+    const int B = a.bins, nj = B * B;
+    const int m0 = v.mq[0] & 255;
+    const int key = v.fb * B + m0;
+    uint32_t q1 = 16777216u;
+    const uint32_t same = (uint32_t) m0 * 0x01010101u;
+    if (v.mq[0] != same || v.mq[1] != same) {
+        const float* l2 = v.w2;
+        const float l1[3] = {1.f - l2[0], 1.f - l2[1], 1.f - l2[2]};
+        const float w[8] = {l1[0] * l1[1] * l1[2], l2[0] * l1[1] * l1[2],
+            l1[0] * l2[1] * l1[2], l2[0] * l2[1] * l1[2],
+            l1[0] * l1[1] * l2[2], l2[0] * l1[1] * l2[2],
+            l1[0] * l2[1] * l2[2], l2[0] * l2[1] * l2[2]};
+        q1 = __float2uint_rn (w[0] * 16777216.f);
+        uint32_t q2 = 0;
+        int m2 = -1;
+#pragma unroll
+        for (int k = 1; k < 8; k++) {
+            const int mk = (v.mq[k >> 2] >> (8 * (k & 3))) & 255;
+            const uint32_t q = __float2uint_rn (w[k] * 16777216.f);
+            if (mk == m0) {
+                q1 += q;
+            } else if (m2 < 0 || mk == m2) {
+                m2 = mk;
+                q2 += q;
+            } else {
+                // a third bin (rare): not to the block's counters, which
+                // take one sum a voxel and bin
+                atomicAdd (a.hist + 2 * B + v.fb * B + mk, (u64) q);
+                atomicAdd (a.hist + B + mk, (u64) q);
+            }
+        }
+        if (m2 >= 0) hist_add (sh, nj, v.fb * B + m2, q2);
+    }
+    if (key != r.key) {
+        if (r.key >= 0) hist_flush<LN_MI_HIST> (sh, B, r);
+        r.key = key;
+        r.s[0] = q1;
+        r.s[1] = 1;
+    } else {
+        r.s[0] += q1;
+        r.s[1] += 1;
+    }
+}
+
+// The warped value with the reference's weight products and sum order
+// (LI_VALUE, src/base/interpolate_macros.h:23-38): products ((w_x w_y) w_z) m,
+// added corner by corner.
+__device__ __forceinline__ float
+line_li_value (const Vox& v)
+{
+    const float* b = v.w2;
+    const float a[3] = {1.f - b[0], 1.f - b[1], 1.f - b[2]};
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const float t = __fmul_rn (__fmul_rn (__fmul_rn (k & 1 ? b[0] : a[0],
+            k & 2 ? b[1] : a[1]), k & 4 ? b[2] : a[2]), v.cr[k]);
+        s = k == 0 ? t : __fadd_rn (s, t);
+    }
+    return s;
 }
 
 template <int MODE, bool AXIS, bool ROI>
@@ -314,10 +544,13 @@ line_kernel (const __grid_constant__ LineArgs a)
     extern __shared__ __align__ (16) uint8_t sm[];
     __shared__ double sh_v[LN_MAX_WARPS];
     __shared__ int sh_n[LN_MAX_WARPS];
-    __shared__ double t_v[32 * LN_MAX_WARPS];      // each thread's own sums
-    __shared__ int t_n[32 * LN_MAX_WARPS];
-    t_v[threadIdx.x] = 0.0;
-    t_n[threadIdx.x] = 0;
+    // each thread's own sums
+    __shared__ double t_v[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
+    __shared__ int t_n[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
+    if (ln_mse (MODE)) {
+        t_v[threadIdx.x] = 0.0;
+        t_n[threadIdx.x] = 0;
+    }
     const BspGeom& g = a.g;
     const int vx = g.vpr[0], vy = g.vpr[1], vz = g.vpr[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -344,6 +577,18 @@ line_kernel (const __grid_constant__ LineArgs a)
     u64* sby = (u64*) (sm + m.by);
     float* sbz = (float*) (sm + m.bz);
     ulonglong2* cz = (ulonglong2*) (sm + m.cz);
+    // after the coefficients: the histograms (low and high halves of the
+    // joint one, fixed counts) or the factor table
+    uint32_t* shist = (uint32_t*) (cz + nz * nj * nkx);
+    float* slut = (float*) shist;
+    const int nh = 2 * a.bins * a.bins + a.bins;
+    if (ln_hist (MODE)) {
+        for (int o = threadIdx.x; o < nh; o += blockDim.x) shist[o] = 0u;
+    }
+    if (MODE == LN_PZ_GRAD) {
+        for (int o = threadIdx.x; o < a.bins * a.bins; o += blockDim.x) slut[o] = a.lut[o];
+    }
+    const float scale = MODE == LN_PZ_GRAD ? a.nvf[1] : 0.f;
     for (int o = threadIdx.x; o < 4 * vx; o += blockDim.x) {
         const float w = a.luts[o];
         sbx[o] = pk (w, w);
@@ -421,7 +666,8 @@ line_kernel (const __grid_constant__ LineArgs a)
             fmaf (lo2 (w01.y), lo2 (c1.y), lo2 (w01.x) * lo2 (c0.y))));
     };
     // adjoint row r leaves the window
-    float* out = a.rows + ((size_t) zr * gridDim.y + blockIdx.y) * a.j * 3 * a.nxs
+    float* out = !ln_adjoint (MODE) ? nullptr
+        : a.rows + ((size_t) zr * gridDim.y + blockIdx.y) * a.j * 3 * a.nxs
         + 32 * xw + lane;
     auto retire = [&] (Row& o) {
         if (col.live) {
@@ -442,6 +688,9 @@ line_kernel (const __grid_constant__ LineArgs a)
     u64 jf2 = pk (i2f_small (g.roi_off[1] + ty0 * vy),
         i2f_small (g.roi_off[1] + ty0 * vy));
     const ulonglong2* wy = (const ulonglong2*) sby;
+    Run run;
+    run.key = -1;
+    int nvox = 0;
     auto tile = [&] (auto rc, int t) {
         constexpr int R = decltype (rc)::value;
         load_row (p[(R + 3) & 3], t + 3);
@@ -451,33 +700,77 @@ line_kernel (const __grid_constant__ LineArgs a)
         int cnt = 0;
         for (int ly = 0; ly < ny; ly++) {
             Vox v;
-            line_load<MODE, AXIS, ROI, R> (a, col, g.roi_off[1] + y0 + ly, jf2, wy + 2 * ly, p, v);
-            line_use<MODE, R> (a, wy + 2 * ly, v, q, scf, cnt);
+            line_load<MODE, AXIS, ROI, R> (a, col, g.roi_off[1] + y0 + ly,
+                jf2, wy + 2 * ly, p, v);
+            if constexpr (ln_mse (MODE)) {
+                line_use<MODE, R> (a, wy + 2 * ly, v, q, scf, cnt);
+            } else if constexpr (MODE == LN_PZ_GRAD) {
+                line_use_pz<AXIS, R> (a, wy + 2 * ly, v, slut, scale, q);
+            } else if constexpr (ln_hist (MODE)) {
+                if (MODE == LN_PZ_HIST) line_use_pz_hist (a, v, shist, run);
+                else line_use_mi_hist (a, v, shist, run);
+                nvox += v.ok ? 1 : 0;
+            } else if (col.live) {
+                if (MODE == LN_WARP) {
+                    a.out[v.fidx] = v.ok ? line_li_value (v) : a.outside;
+                } else {
+                    float* o = a.out + 3 * (size_t) v.fidx;
+                    o[0] = v.cr[0];
+                    o[1] = v.cr[1];
+                    o[2] = v.cr[2];
+                }
+            }
         }
-        t_v[threadIdx.x] += (double) scf;
-        t_n[threadIdx.x] += cnt;
-        retire (q[R]);
+        if (ln_mse (MODE)) {
+            t_v[threadIdx.x] += (double) scf;
+            t_n[threadIdx.x] += cnt;
+        }
+        if (ln_adjoint (MODE)) retire (q[R]);
     };
     if (wlive) {
-    load_row (p[0], 0);
-    load_row (p[1], 1);
-    load_row (p[2], 2);
-    for (int t = 0; t < nt; t++) {
-        switch (t & 3) {
-        case 0: tile (std::integral_constant<int, 0> (), t); break;
-        case 1: tile (std::integral_constant<int, 1> (), t); break;
-        case 2: tile (std::integral_constant<int, 2> (), t); break;
-        default: tile (std::integral_constant<int, 3> (), t); break;
+        load_row (p[0], 0);
+        load_row (p[1], 1);
+        load_row (p[2], 2);
+        for (int t = 0; t < nt; t++) {
+            switch (t & 3) {
+            case 0: tile (std::integral_constant<int, 0> (), t); break;
+            case 1: tile (std::integral_constant<int, 1> (), t); break;
+            case 2: tile (std::integral_constant<int, 2> (), t); break;
+            default: tile (std::integral_constant<int, 3> (), t); break;
+            }
+        }
+        // the three rows that are left in the window
+        if (ln_adjoint (MODE)) {
+            switch (nt & 3) {
+            case 0: retire (q[0]); retire (q[1]); retire (q[2]); break;
+            case 1: retire (q[1]); retire (q[2]); retire (q[3]); break;
+            case 2: retire (q[2]); retire (q[3]); retire (q[0]); break;
+            default: retire (q[3]); retire (q[0]); retire (q[1]); break;
+            }
         }
     }
-    // the three rows that are left in the window
-    switch (nt & 3) {
-    case 0: retire (q[0]); retire (q[1]); retire (q[2]); break;
-    case 1: retire (q[1]); retire (q[2]); retire (q[3]); break;
-    case 2: retire (q[2]); retire (q[3]); retire (q[0]); break;
-    default: retire (q[3]); retire (q[0]); retire (q[1]); break;
+    if constexpr (ln_hist (MODE)) {
+        const int B = a.bins;
+        if (run.key >= 0) hist_flush<MODE> (shist, B, run);
+        nvox = __reduce_add_sync (0xffffffffu, nvox);
+        if (lane == 0 && nvox) atomicAdd (a.hist + 2 * B + B * B, (u64) nvox);
+        __syncthreads ();
+        for (int o = threadIdx.x; o < B * B; o += blockDim.x) {
+            const u64 w = (u64) shist[o] + ((u64) shist[B * B + o] << 16);
+            if (w) {
+                atomicAdd (a.hist + 2 * B + o, w);
+                // the moving histogram: the joint one's column sums
+                if (MODE == LN_MI_HIST) atomicAdd (a.hist + B + o % B, w);
+            }
+        }
+        if (MODE == LN_MI_HIST) {
+            for (int o = threadIdx.x; o < B; o += blockDim.x) {
+                const uint32_t w = shist[2 * B * B + o];
+                if (w) atomicAdd (a.hist + o, (u64) w);
+            }
+        }
     }
-    }
+    if constexpr (ln_mse (MODE)) {
 
     // the block's score and count, in warp order
     double sc = t_v[threadIdx.x];
@@ -502,6 +795,7 @@ line_kernel (const __grid_constant__ LineArgs a)
         const int b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
         a.score_part[b] = v;
         a.count_part[b] = n;
+    }
     }
 }
 
@@ -797,7 +1091,9 @@ line_plan (const BspGeom& g, LinePlan* p, int sm_count)
         const double cost = (double) per_sm * (ty + LN_EDGE / g.vpr[1])
             / rate[std::min<long long> (per_sm, 4)];
         const LineSmem m = line_smem (g.vpr[0], g.vpr[1], g.vpr[2], ty + 3, foot);
-        if (p->ty && (m.total > 48 * 1024 || cost >= best)) continue;
+        // (fewer than 65536 voxels a block: its histogram counters)
+        if (p->ty && (m.total > 48 * 1024 || cost >= best
+                || p->nw * 32 * ty * g.vpr[1] > 65535)) continue;
         best = cost;
         p->ty = ty;
         p->nys = nys;
@@ -823,10 +1119,13 @@ axis_aligned (const BspGeom& g)
 }
 
 static void
-line_args (const BspGeom& g, const LinePlan& p, LineArgs& a)
+line_args (const BspGeom& g, const LinePlan& p, const float* coeff,
+    const float* luts, LineArgs& a)
 {
     a = LineArgs ();
     a.g = g;
+    a.coeff = coeff;
+    a.luts = luts;
     a.ty = p.ty;
     a.j = p.j;
     a.nxs = p.nxs;
@@ -850,26 +1149,31 @@ launch (const LinePlan& p, const LineArgs& a, cudaStream_t st)
 {
     const BspGeom& g = a.g;
     auto k = line_kernel<MODE, AXIS, ROI>;
-    if (p.smem > 48 * 1024) {
-        cudaError_t e = set_max_dynamic_smem ((const void*) k, (int) p.smem);
+    size_t smem = p.smem;
+    if (ln_hist (MODE)) smem += (2 * a.bins * a.bins + a.bins) * sizeof (uint32_t);
+    if (MODE == LN_PZ_GRAD) smem += a.bins * a.bins * sizeof (float);
+    if (smem > 48 * 1024) {
+        cudaError_t e = set_max_dynamic_smem ((const void*) k, (int) smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<dim3 (p.gpr, p.nys, g.rdims[2]), p.threads, p.smem, st>>> (a);
+    k<<<dim3 (p.gpr, p.nys, g.rdims[2]), p.threads, smem, st>>> (a);
     return cudaGetLastError ();
 }
 
 template <int MODE>
 static cudaError_t
-launch_mode (const BspGeom& g, const LinePlan& p, const LineArgs& a,
-    cudaStream_t st)
+launch_mode (const LinePlan& p, const LineArgs& a, cudaStream_t st)
 {
-    const bool roi = g.fmask || g.mroi;
-    if (axis_aligned (g)) {
-        return roi ? launch<MODE, true, true> (p, a, st)
-                   : launch<MODE, true, false> (p, a, st);
+    const BspGeom& g = a.g;
+    const bool axis = axis_aligned (g);
+    if constexpr (ln_mse (MODE)) {
+        if (g.fmask || g.mroi) {
+            return axis ? launch<MODE, true, true> (p, a, st)
+                        : launch<MODE, false, true> (p, a, st);
+        }
     }
-    return roi ? launch<MODE, false, true> (p, a, st)
-               : launch<MODE, false, false> (p, a, st);
+    return axis ? launch<MODE, true, false> (p, a, st)
+                : launch<MODE, false, false> (p, a, st);
 }
 
 cudaError_t
@@ -879,19 +1183,77 @@ launch_mse_line (const BspGeom& g, const LinePlan& p, int grad_mode,
     int* count_part, cudaStream_t st)
 {
     LineArgs a;
-    line_args (g, p, a);
+    line_args (g, p, coeff, luts, a);
     a.fimg = fimg;
     a.mimg = mimg;
     a.mgrad4 = mgrad4;
-    a.coeff = coeff;
-    a.luts = luts;
     a.rows = rows;
     a.score_part = score_part;
     a.count_part = count_part;
-    return grad_mode == 0 ? launch_mode<LN_MSE_NEAREST> (g, p, a, st)
-                          : launch_mode<LN_MSE_LINEAR> (g, p, a, st);
+    return grad_mode == 0 ? launch_mode<LN_MSE_NEAREST> (p, a, st)
+                          : launch_mode<LN_MSE_LINEAR> (p, a, st);
 }
 
+cudaError_t
+launch_mi_line (const BspGeom& g, const LinePlan& p, bool hist_pass,
+    const LineMi& mi, const float* coeff, const float* luts, float* rows,
+    cudaStream_t st)
+{
+    LineArgs a;
+    line_args (g, p, coeff, luts, a);
+    a.fbin = mi.fbin;
+    a.mquad = mi.mquad;
+    a.bins = mi.bins;
+    a.lut = mi.lut;
+    a.nvf = mi.nvf;
+    a.hist = mi.hist;
+    a.mimg = mi.mimg;
+    a.pz_min = mi.m_min;
+    a.pz_inv = 1.f / mi.m_delta;
+    a.rows = rows;
+    if (!mi.parzen) {
+        return hist_pass ? launch_mode<LN_MI_HIST> (p, a, st) : cudaErrorInvalidValue;
+    }
+    return hist_pass ? launch_mode<LN_PZ_HIST> (p, a, st)
+                     : launch_mode<LN_PZ_GRAD> (p, a, st);
+}
+
+cudaError_t
+launch_field_line (const BspGeom& g, const LinePlan& p, const float* coeff,
+    const float* luts, const float* mimg, float outside, float* vf,
+    float* warped, cudaStream_t st)
+{
+    LineArgs a;
+    line_args (g, p, coeff, luts, a);
+    a.mimg = mimg;
+    a.outside = outside;
+    a.out = vf ? vf : warped;
+    return vf ? launch_mode<LN_FIELD> (p, a, st) : launch_mode<LN_WARP> (p, a, st);
+}
+
+// Bins of the 2 x 2 moving voxels from each voxel on (x fastest, a byte
+// each): one 4-byte load in place of four of one byte.
+__global__ void
+bin_quad_kernel (int nx, int ny, long long n, const uint8_t* __restrict__ bin,
+    uint32_t* __restrict__ quad)
+{
+    for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (long long) gridDim.x * blockDim.x) {
+        const int x = (int) (i % nx), y = (int) ((i / nx) % ny);
+        const int dx = x + 1 < nx ? 1 : 0, dy = y + 1 < ny ? nx : 0;
+        quad[i] = bin[i] | (uint32_t) bin[i + dx] << 8
+            | (uint32_t) bin[i + dy] << 16 | (uint32_t) bin[i + dy + dx] << 24;
+    }
+}
+
+cudaError_t
+launch_bin_quad (const int dim[3], const uint8_t* bin, uint32_t* quad,
+    cudaStream_t st)
+{
+    bin_quad_kernel<<<1184, 256, 0, st>>> (dim[0], dim[1],
+        (long long) dim[0] * dim[1] * dim[2], bin, quad);
+    return cudaGetLastError ();
+}
 
 cudaError_t
 launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,

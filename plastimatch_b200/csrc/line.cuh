@@ -33,6 +33,31 @@ cudaError_t launch_mse_line (const BspGeom& g, const LinePlan& p,
     const float4* mgrad4, const float* coeff, const float* luts, float* rows,
     double* score_part, int* count_part, cudaStream_t st);
 
+// Mattes MI: pass 1 (PVI-8 or Parzen histograms into hist, integer 2^-24
+// units, count last) or, for Parzen windows, pass 2 (adjoint rows).
+struct LineMi {
+    const uint8_t* fbin;
+    const uint32_t* mquad;       // PVI-8: launch_bin_quad's image
+    int bins;
+    const float* lut;            // Parzen pass 2: [fixed bin][moving bin]
+    const float* nvf;            //   [1]: 1 / (N delta_m)
+    unsigned long long* hist;    // f[B], m[B], j[B*B], count
+    bool parzen;
+    const float* mimg;           // Parzen: the moving image
+    float m_min, m_delta;        // Parzen: moving value -> window centre
+};
+cudaError_t launch_mi_line (const BspGeom& g, const LinePlan& p,
+    bool hist_pass, const LineMi& mi, const float* coeff, const float* luts,
+    float* rows, cudaStream_t st);
+cudaError_t launch_bin_quad (const int dim[3], const uint8_t* bin,
+    uint32_t* quad, cudaStream_t st);
+
+// Dense field (vf) or warped moving image (warped; the other is NULL) over
+// the ROI's voxels.
+cudaError_t launch_field_line (const BspGeom& g, const LinePlan& p,
+    const float* coeff, const float* luts, const float* mimg, float outside,
+    float* vf, float* warped, cudaStream_t st);
+
 // Contraction of the adjoint rows into the gradient, score and count over
 // the nparts block parts (0: the result block stands, no normalisation), as
 // launch_finish_mse otherwise.

@@ -26,6 +26,7 @@
 
 #include "../../include/plastimatch_b200.h"
 #include "fp32_tile.cuh"
+#include "line.cuh"
 #include "mi.cuh"
 
 namespace b200 {
@@ -275,6 +276,18 @@ mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist)
     return B200BSP_OK;
 }
 
+int
+mi_alloc_line (MiState* s, const BspGeom& g)
+{
+    const size_t nm = (size_t) g.mdim[0] * g.mdim[1] * g.mdim[2];
+    if (s->window != B200BSP_MI_PVI8) return B200BSP_OK;
+    if (cudaMalloc (&s->d_mquad, nm * sizeof (uint32_t)) != cudaSuccess) {
+        cudaGetLastError ();
+        return B200BSP_E_OOM;
+    }
+    return B200BSP_OK;
+}
+
 void
 mi_free (MiState* s)
 {
@@ -283,6 +296,7 @@ mi_free (MiState* s)
     cudaFree (s->d_minmax); cudaFree (s->d_part); cudaFree (s->d_score_part);
     cudaFree (s->d_count_part);
     cudaFree (s->d_fkey); cudaFree (s->d_mkey);
+    cudaFree (s->d_mquad);
     cudaFreeHost (s->h_histd); cudaFreeHost (s->h_res);
     *s = MiState ();
 }
@@ -313,6 +327,10 @@ mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
             s->d_fkey, s->d_fbin, st);
         if (!rc) rc = vopt_bins (d_moving, nm, s->bins, &s->m_offset,
             &s->m_delta, s->d_mkey, s->d_mbin, st);
+        if (!rc && s->d_mquad && launch_bin_quad (g.mdim, s->d_mbin,
+                s->d_mquad, st) != cudaSuccess) {
+            rc = B200BSP_E_CUDA;
+        }
         if (rc) return rc;
         s->ready = true;
         return B200BSP_OK;
@@ -327,6 +345,7 @@ mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
         s->f_offset, s->f_delta, s->bins, s->d_fbin);
     bin_image_kernel<<<1184, 256, 0, st>>> (d_moving, (long long) nm,
         s->m_offset, s->m_delta, s->bins, s->d_mbin);
+    if (s->d_mquad) launch_bin_quad (g.mdim, s->d_mbin, s->d_mquad, st);
     if (cudaGetLastError () != cudaSuccess) return B200BSP_E_CUDA;
     s->ready = true;
     return B200BSP_OK;
@@ -994,6 +1013,51 @@ mi_run_xl (MiState* s, const BspGeom& g, const XlPlan& plan,
     }
     if (launches) *launches += 4;
     return cudaGetLastError () == cudaSuccess ? B200BSP_OK : B200BSP_E_CUDA;
+}
+
+// Pass 1 and, for Parzen windows, the score and pass 2 on the line kernel.
+int
+mi_run_line (MiState* s, const BspGeom& g, const LinePlan& plan,
+    float* rows, const float* d_coeff, const float* d_moving,
+    const float* d_luts, DevResult* d_res, float* grad_out,
+    double* grad64_out, cudaStream_t st, int* launches, int passes)
+{
+    if (!s->ready) return B200BSP_E_STATE;
+    const int B = s->bins;
+    const int nh = 2 * B + B * B;
+    LineMi mi;
+    mi.fbin = s->d_fbin;
+    mi.mquad = s->d_mquad;
+    mi.bins = B;
+    mi.lut = s->d_lut;
+    mi.nvf = s->d_nvf;
+    mi.hist = s->d_hist;
+    mi.parzen = s->window == B200BSP_MI_PARZEN;
+    mi.mimg = d_moving;
+    mi.m_min = s->pz_mmin;
+    mi.m_delta = s->pz_mdelta;
+    if (passes & MI_PASS_HIST) {
+        if (cudaMemsetAsync (s->d_hist, 0, (nh + 1) * sizeof (unsigned long long),
+                st) != cudaSuccess
+            || launch_mi_line (g, plan, true, mi, d_coeff, d_luts, nullptr, st)
+                != cudaSuccess) {
+            return B200BSP_E_CUDA;
+        }
+        if (launches) *launches += 1;
+    }
+    if (!(passes & MI_PASS_GRAD)) return B200BSP_OK;
+    parzen_score_kernel<<<1, 1024, 0, st>>> (s->d_hist, B, s->pz_mdelta,
+        s->d_histd, s->d_lut, s->d_nvf, d_res);
+    if (cudaGetLastError () != cudaSuccess
+        || launch_mi_line (g, plan, false, mi, d_coeff, d_luts, rows, st)
+            != cudaSuccess
+        || launch_line_finish (g, plan, rows, d_luts, nullptr, nullptr, 0,
+            nullptr, d_res, nullptr, grad_out, grad64_out, nullptr, nullptr,
+            nullptr, st) != cudaSuccess) {
+        return B200BSP_E_CUDA;
+    }
+    if (launches) *launches += 3;
+    return B200BSP_OK;
 }
 
 int

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
+#include "line.cuh"
 
 namespace b200 {
 
@@ -34,6 +35,7 @@ struct MiState {
     float f_offset = 0.f, f_delta = 1.f, m_offset = 0.f, m_delta = 1.f;
     uint8_t* d_fbin = nullptr;                // fixed-image bin per voxel
     uint8_t* d_mbin = nullptr;                // moving-image bin per voxel
+    uint32_t* d_mquad = nullptr;              // line kernel: bins of 2 x 2 voxels
     unsigned long long* d_hist = nullptr;     // f[B], m[B], j[B*B], N (fixed point)
     double* d_histd = nullptr;                // f, m, j as doubles
     float* d_lut = nullptr;                   // dS/dP per joint bin (0 = skip)
@@ -49,6 +51,8 @@ struct MiState {
 
 int mi_alloc (MiState* s, const BspGeom& g, int bins, int window,
     int hist = 0);
+// The line kernel's bin image (contexts that may run it).
+int mi_alloc_line (MiState* s, const BspGeom& g);
 void mi_free (MiState* s);
 int mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
     const float* d_moving, size_t nf, size_t nm, cudaStream_t st);
@@ -71,6 +75,10 @@ int mi_run_xl (MiState* s, const BspGeom& g, const XlPlan& plan,
     const float* d_moving, DevResult* d_res, float* grad_out,
     double* grad64_out, cudaStream_t st, int* launches,
     int passes = MI_PASS_HIST | MI_PASS_GRAD);
+int mi_run_line (MiState* s, const BspGeom& g, const LinePlan& plan,
+    float* rows, const float* d_coeff, const float* d_moving,
+    const float* d_luts, DevResult* d_res, float* grad_out,
+    double* grad64_out, cudaStream_t st, int* launches, int passes);
 int mi_fetch (MiState* s, const DevResult* d_res, double* f_hist,
     double* m_hist, double* j_hist, cudaStream_t st);
 void mi_finish (MiState* s, MiResult* r);

@@ -37,6 +37,7 @@ void* ctx_opt_ws (const b200bsp_ctx* c);
 int ctx_landmarks (const b200bsp_ctx* c, float* stiffness);
 void ctx_set_opt_ws (b200bsp_ctx* c, void* ws, void (*release) (void*));
 unsigned ctx_generation (const b200bsp_ctx* c);                // runtime.cu
+void ctx_hold_line (b200bsp_ctx* c, int by);
 int* ctx_err_flag (b200bsp_ctx* c);
 int ctx_report_device_error (b200bsp_ctx* c, int e);
 
@@ -1312,7 +1313,10 @@ b200bsp_optimize_lbfgs (b200bsp_ctx* ctx, int metric_type, float lambda,
     if (rc) return rc;
     ContextObjective obj;
     obj.ctx = ctx; obj.metric = metric_type; obj.lambda = lambda; obj.reg = reg;
-    return optimize_on_context (ctx, p, nc, coeff, res, obj);
+    ctx_hold_line (ctx, 1);
+    rc = optimize_on_context (ctx, p, nc, coeff, res, obj);
+    ctx_hold_line (ctx, -1);
+    return rc;
 }
 
 extern "C" int

@@ -79,6 +79,7 @@ struct b200bsp_ctx {
     // the line kernel (line.cu), an AUTO context's choice on the grids that
     // line_plan takes
     bool use_line = false;
+    int line_hold = 0;        // > 0 inside the optimiser and the autotuner
     LinePlan lplan;
     float* d_rows = nullptr;
     // b200bsp_score's device path: the regulariser on a second stream,
@@ -405,6 +406,17 @@ ctx_landmarks (const b200bsp_ctx* c, float* stiffness)
     return c->lm_n;
 }
 
+// Evaluations between ctx_hold_line (c, 1) and (c, -1) stay on the kernels
+// that the context runs without the line kernel.  The optimiser takes them:
+// its iterates amplify the last bits of the gradient (by a factor of 100 to
+// 1000 within four iterations, through the differences of gradients that it
+// divides by), so a registration keeps its path only on one kernel.
+void
+ctx_hold_line (b200bsp_ctx* c, int by)
+{
+    c->line_hold += by;
+}
+
 unsigned
 ctx_generation (const b200bsp_ctx* c)
 {
@@ -682,6 +694,9 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
             o.mi_hist)) {
         rc2 = fail (c, B200BSP_E_OOM, "MI buffers: out of device memory");
     }
+    if (!rc2 && c->use_line && mi_alloc_line (&c->mi, c->geom)) {
+        rc2 = fail (c, B200BSP_E_OOM, "MI buffers: out of device memory");
+    }
     if (!rc2) {
         // Bspline_xform::grid_spac = vox_per_rgn * |spacing| (float)
         float gsp[3];
@@ -749,8 +764,7 @@ b200bsp_set_wait_limit (b200bsp_ctx* c, int polls, int withhold_mma)
 {
     if (!c) return B200BSP_E_BADARG;
     if (polls < 0) return fail (c, B200BSP_E_BADARG, "polls must be >= 0");
-    if (withhold_mma && !(c->opts.form == B200BSP_FORM_TC && c->use_xl
-            && !c->use_line)) {
+    if (withhold_mma && !(c->opts.form == B200BSP_FORM_TC && c->use_xl)) {
         return fail (c, B200BSP_E_UNSUPPORTED,
             "withholding MMAs is a testing aid of the x-lane kernel");
     }
@@ -898,6 +912,13 @@ end_eval (b200bsp_ctx* c, bool wait)
     return B200BSP_OK;
 }
 
+// Whether the next evaluation runs on the line kernel.
+static bool
+line_now (const b200bsp_ctx* c)
+{
+    return c->use_line && c->line_hold == 0;
+}
+
 // The MSE tile pass + reductions, results left in d_res and the given
 // gradient outputs (device pointers).
 static int
@@ -913,7 +934,7 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
         CK (launch_mse_fp32 (g, c->opts.mse_grad, c->d_fixed, c->d_moving,
             c->d_mgrad, dcoeff, c->d_luts, c->d_part, c->d_score_part,
             c->d_count_part, c->stream));
-    } else if (c->use_line) {
+    } else if (line_now (c)) {
         CK (launch_mse_line (g, c->lplan, c->opts.mse_grad, c->d_fixed,
             c->d_moving, c->d_mgrad4, dcoeff, c->d_luts, c->d_rows,
             c->d_score_part, c->d_count_part, c->stream));
@@ -945,7 +966,7 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
     }
     const bool xl = c->opts.form == B200BSP_FORM_TC && c->use_xl;
     if (before_finish) CK (cudaStreamWaitEvent (c->stream, before_finish, 0));
-    if (c->use_line) {
+    if (line_now (c)) {
         CK (launch_line_finish (g, c->lplan, c->d_rows, c->d_luts,
             c->d_score_part, c->d_count_part, c->lplan.nblocks, c->d_err,
             c->d_res, res_host, grad_out, grad64_out, score_out, score64_out,
@@ -1058,17 +1079,13 @@ b200bsp_autotune (b200bsp_ctx* c, const float* coeff, int evals, int* tiles)
     const float* dcoeff = nullptr;
     int rc = begin_eval (c, coeff, &dcoeff);
     if (rc) return rc;
-    if (c->use_line) {
-        // its plan follows from the grid: nothing to choose
-        if (tiles) *tiles = c->lplan.kx;
-        return B200BSP_OK;
-    }
     int sm_count = 148;
     cudaDeviceGetAttribute (&sm_count, cudaDevAttrMultiProcessorCount,
         c->device);
     cudaEvent_t e0, e1;
     CK (cudaEventCreate (&e0));
     CK (cudaEventCreate (&e1));
+    c->line_hold++;
     const TcPlan start = c->plan;
     const bool start_xl = c->use_xl;
     TcPlan best = start;
@@ -1122,6 +1139,7 @@ b200bsp_autotune (b200bsp_ctx* c, const float* coeff, int evals, int* tiles)
             best_xl = false;
         }
     }
+    c->line_hold--;
     cudaEventDestroy (e0);
     cudaEventDestroy (e1);
     use_tc_plan (c, rc ? start : best);
@@ -1168,6 +1186,23 @@ mi_passes_on (b200bsp_ctx* c, const BspGeom& g, const float* dcoeff,
     float* grad, double* grad64, int passes)
 {
     const bool roi = g.fmask || g.mroi;
+    // The line kernel takes Parzen windows' passes and PVI-8's pass 1.
+    // PVI-8's gradient jumps wherever a position crosses a cell's face, so
+    // its pass 2 stays with the field it has always been formed from.
+    if (line_now (c) && !roi) {
+        const bool parzen = c->opts.mi_window == B200BSP_MI_PARZEN;
+        const int now = parzen ? passes : passes & MI_PASS_HIST;
+        LinePlan p = c->lplan;
+        bool ok = now != 0;
+        if (ok && &g != &c->geom) ok = line_plan (g, &p, c->sm_count);
+        if (ok) {
+            const int rc = mi_run_line (&c->mi, g, p, c->d_rows, dcoeff,
+                c->d_moving, c->d_luts, c->d_res, grad, grad64, c->stream,
+                &c->last_launches, now);
+            passes &= ~now;
+            if (rc || !passes) return rc;
+        }
+    }
     // the tile kernel's MI passes are the faster ones where both apply
     // (PVI-8, 32 bins, 256x256x128 at vpr 5: 332 + 179 us against 532 +
     // 223 us); the x-lane kernel's when pinned or the tile kernel cannot
@@ -1838,8 +1873,16 @@ field_warp (b200bsp_ctx* c, const float* coeff, float* vf, float* warped,
         whole = whole && g.roi_off[d] == 0 && g.roi_dim[d] == g.fdim[d];
     }
     if (vf && !whole) CK (cudaMemsetAsync (target, 0, bytes, c->stream));
-    CK (launch_field_warp (g, dcoeff, c->d_luts, c->d_moving, default_value,
-        vf ? target : nullptr, vf ? nullptr : target, c->stream));
+    LinePlan p;
+    if (line_plan (g, &p, c->sm_count)) {
+        CK (launch_field_line (g, p, dcoeff, c->d_luts, c->d_moving,
+            default_value, vf ? target : nullptr, vf ? nullptr : target,
+            c->stream));
+    } else {
+        CK (launch_field_warp (g, dcoeff, c->d_luts, c->d_moving,
+            default_value, vf ? target : nullptr, vf ? nullptr : target,
+            c->stream));
+    }
     c->last_launches = 1;
     rc = mark_main_done (c);
     if (rc) return rc;

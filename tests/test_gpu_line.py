@@ -78,3 +78,62 @@ def test_regions_outside_the_line_kernel_keep_the_tile_kernel():
     for vpr in ((5, 12, 5), (2, 5, 5), (5, 5, 11)):
         with P.Context(f, f, BsplineGrid.for_volume(f, vpr)) as ctx:
             assert ctx.mse_kernel()[0] == "tile"
+
+
+@pytest.mark.parametrize("window,bins", [("pvi8", 20), ("pvi8", 64),
+                                         ("parzen", 32), ("parzen", 5)])
+@pytest.mark.parametrize("case", [c for c in CASES if c[2] is None])
+def test_line_kernel_mi_matches_tile_kernel(case, window, bins):
+    """Mattes MI: the line kernel's histograms (and, for Parzen windows, its
+    gradient) against the FP32 form's.  The weights are sums of 2^-24 units of
+    positions that agree to some 2^-21 voxel, so the histograms agree to 1e-6
+    of their counts times the few voxels per bin edge: bar 1e-5; the score, a
+    sum over them, 1e-5; the Parzen gradient, whose window derivative scales
+    the same differences by at most 2 bins, 5e-5."""
+    fixed, moving, grid, coeff = _case(*case)
+    out = []
+    for form in ("fp32", "tc"):
+        with P.Context(fixed, moving, grid, form=form, mi_window=window,
+                       mi_bins=bins) as ctx:
+            ctx.set_images()
+            out.append(ctx.score_mi(coeff, with_hist=True))
+            h = ctx.mi_hist(coeff)
+            np.testing.assert_array_equal(h, ctx.mi_hist(coeff))
+            assert h[-1] == out[-1][2]
+            if window == "pvi8":       # every voxel once, eight weights each
+                assert h[:bins].sum() == h[-1]
+                assert h[bins:2 * bins].sum() == h[2 * bins:-1].sum()
+    (s0, g0, n0, h0), (s1, g1, n1, h1) = out
+    assert n0 > 0 and abs(n1 - n0) <= 1e-4 * n0 + 2, (n1, n0)
+    for a, b in zip(h1, h0):
+        assert rel_err(a, b) < 1e-5 + 2.0 / n0, rel_err(a, b)
+    assert abs(s1 - s0) <= 1e-5 * abs(s0) + 1e-6, (s1, s0)
+    if window == "parzen":
+        assert rel_err(g1, g0) < 5e-5, rel_err(g1, g0)
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_line_kernel_field_and_warp(case):
+    """The dense field against its double-precision evaluation (64 products
+    of coefficients up to some 6 mm: 1e-5 mm), and the warp against the
+    trilinear sample at those positions (1e-3 of the image's 1000 grey levels
+    times a position error of 1e-4 voxel, away from the image's edge)."""
+    fixed, moving, grid, coeff = _case(*case)
+    off, dim = grid.roi_offset, grid.roi_dim
+    roi = tuple(slice(off[d], off[d] + dim[d]) for d in (2, 1, 0))
+    ref = synth.bspline_field(grid, coeff)
+    for form in ("fp32", "tc"):
+        with P.Context(fixed, moving, grid, form=form) as ctx:
+            ctx.set_images()
+            vf = ctx.interpolate_vf(coeff)
+            np.testing.assert_allclose(vf[roi], ref, atol=1e-5)
+            mask = np.ones(vf.shape[:3], bool)
+            mask[roi] = False
+            assert not vf[mask].any()
+            if case[2] is not None:
+                continue
+            w = ctx.warp(coeff, -7.0)
+    if case[2] is None:
+        want = synth.warp_trilinear(moving, fixed, grid, coeff, -7.0).img
+        bad = np.abs(w - want) > 0.1
+        assert bad.mean() < 1e-4, bad.mean()
