@@ -18,17 +18,18 @@
 // run in an order of their own: results do not depend on how blocks are
 // scheduled.
 //
-// Measured at 256x256x128, 5 voxels a region, nearest gradient: 75 us and 11
+// Measured at 256x256x128, 5 voxels a region, nearest gradient: 67 us and 13
 // us for the contraction, where the tcgen05 tile kernel takes 160 and 7 us
-// (64x64x64, 8 voxels: 8 + 9 against 22 + 5 us; 512x512x160, 10x10x4: 346 +
-// 43 against 800 + 40 us).  The tensor cores' field must be carried through
+// (64x64x64, 8 voxels: 8 + 9 against 22 + 5 us; 512x512x160, 10x10x4: 316 +
+// 36 against 800 + 40 us).  The tensor cores' field must be carried through
 // shared memory to the x order and their adjoint operand split into bf16
 // pairs, which costs more instructions than 24 two-wide multiply-adds.
-// What bounds it: issue.  150 instructions a voxel, of which some 60 are
-// address and clamp arithmetic, at 48 % of the issue slots; without any load
-// 47 us, with loads that all hit L1 58 us.  Prefetching the next rows into L2
-// or L1, or loading a voxel ahead, changes nothing (within 2 %): the misses
-// are hidden by the other 31 warps.
+// What bounds it: 147 instructions a voxel, some 60 of them address and clamp
+// arithmetic, at half the issue slots, and the latency of the loads between
+// them.  Without any load 47 us, with loads that all hit L1 58 us.
+// Prefetching the next rows into L2 or L1, loading a voxel ahead, corners by
+// texture gather (105 us) or the gradient from the moving image instead of
+// memory (86 us) do not help.
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -38,6 +39,8 @@
 #include "line.cuh"
 
 namespace b200 {
+
+void basis_lut (float* lut, int vpr);               // runtime.cu
 
 // What a block does at each voxel: MSE with the nearest or the trilinear
 // moving gradient; Mattes MI pass 1 (PVI-8 or Parzen histograms) and, for
@@ -67,6 +70,9 @@ ln_adjoint (int mode)
 }
 
 constexpr int LN_MAX_WARPS = 16;
+// dynamic shared memory that needs no attribute beside the static arrays
+constexpr size_t LN_PLAIN_SMEM = 40 * 1024;
+constexpr int LN_MAX_VPR = 10;           // voxels a region (line_plan)
 constexpr int LN_REGS = 64;             // four blocks of eight warps per SM
 constexpr int LN_WARPS = 8;             // warps a block (see line_plan)
 constexpr double LN_EDGE = 2.5;         // a block's start and end, in voxels
@@ -77,7 +83,7 @@ struct LineArgs {
     BspGeom g;
     const float* fimg;
     const float* mimg;
-    const float4* mgrad4;
+    const float* mgrad;  // xyz interleaved
     const float* coeff;
     const float* luts;
     float* rows;         // adjoint rows [z][y block][j][c][nxs]
@@ -93,6 +99,11 @@ struct LineArgs {
     float* out;          // field (xyz per voxel) or warped image
     float outside;
     int ty, j, nxs;
+    // y weights of each row of a tile, each twice; in the parameter bank,
+    // since they are the same for every thread: shared memory would return
+    // them to all 32 lanes (four cycles a 16-byte load: 44 instead of 31 L1
+    // cycles a voxel, and 8 registers that then spill: 75 against 70 us)
+    u64 wy[LN_MAX_VPR][4];
     u64 step_y;          // AXIS: (0, fixed y step)
     u64 morg, mprj;      // AXIS: moving x and y origin and projection
     int mtop[3];         // bits of 2^23 + (dim - 2): the largest corner
@@ -159,17 +170,16 @@ struct Row {
 
 // Shared memory of a block, in bytes from its start.
 struct LineSmem {
-    int bx, by, bz, cz, total;
+    int bx, bz, cz, total;
 };
 
 // cz: planes x knots of a block's footprint (line_foot), times its rows.
 __host__ __device__ inline LineSmem
-line_smem (int vx, int vy, int vz, int j, int foot)
+line_smem (int vx, int vz, int j, int foot)
 {
     LineSmem m;
     m.bx = 0;
-    m.by = m.bx + 32 * vx;
-    m.bz = m.by + 32 * vy;
+    m.bz = m.bx + 32 * vx;
     m.cz = m.bz + 16 * vz;
     m.total = m.cz + 16 * j * foot;
     return m;
@@ -188,7 +198,7 @@ struct Col {
 // One voxel between its loads and its metric.
 struct Vox {
     float cr[8], fv;
-    float4 gr;
+    float gr[3];
     float w2[3];
     uint32_t mq[2];
     int fb, fidx, clamp;
@@ -205,32 +215,23 @@ ld1 (const float* p)
     return v;
 }
 
-__device__ __forceinline__ float4
-ld4 (const float4* p)
-{
-    float4 v;
-    asm volatile ("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-        : "=f" (v.x), "=f" (v.y), "=f" (v.z), "=f" (v.w) : "l" (p));
-    return v;
-}
-
-// The voxel at fixed row fj (y weights wy): field, correspondence, loads.
+// The voxel at fixed row fj (row ly of its tile): field, correspondence, loads.
 // R: the window's first slot.
 template <int MODE, bool AXIS, bool ROI, int R>
 __device__ __forceinline__ void
 line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
-    const ulonglong2* __restrict__ wy, const Row (&p)[4], Vox& v)
+    int ly, const Row (&p)[4], Vox& v)
 {
     const BspGeom& g = a.g;
-    const ulonglong2 w01 = wy[0], w23 = wy[1];
-    u64 dxy = mul2 (w01.x, p[R].xy);
-    dxy = fma2 (w01.y, p[(R + 1) & 3].xy, dxy);
-    dxy = fma2 (w23.x, p[(R + 2) & 3].xy, dxy);
-    dxy = fma2 (w23.y, p[(R + 3) & 3].xy, dxy);
-    float dz = lo2 (w01.x) * p[R].z;
-    dz = fmaf (lo2 (w01.y), p[(R + 1) & 3].z, dz);
-    dz = fmaf (lo2 (w23.x), p[(R + 2) & 3].z, dz);
-    dz = fmaf (lo2 (w23.y), p[(R + 3) & 3].z, dz);
+    const u64* w = a.wy[ly];
+    u64 dxy = mul2 (w[0], p[R].xy);
+    dxy = fma2 (w[1], p[(R + 1) & 3].xy, dxy);
+    dxy = fma2 (w[2], p[(R + 2) & 3].xy, dxy);
+    dxy = fma2 (w[3], p[(R + 3) & 3].xy, dxy);
+    float dz = lo2 (w[0]) * p[R].z;
+    dz = fmaf (lo2 (w[1]), p[(R + 1) & 3].z, dz);
+    dz = fmaf (lo2 (w[2]), p[(R + 2) & 3].z, dz);
+    dz = fmaf (lo2 (w[3]), p[(R + 3) & 3].z, dz);
     const float jf = lo2 (jf2);
     float fx[3];
     float ma[3];
@@ -302,7 +303,10 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
     if (MODE == LN_MSE_NEAREST) {
         const int mvr = mvf + (v.w2[0] >= 0.5f ? 1 : 0)
             + (v.w2[1] >= 0.5f ? dx : 0) + (v.w2[2] >= 0.5f ? dxym : 0);
-        v.gr = ld4 (a.mgrad4 + mvr);
+        const float* gp = a.mgrad + 3 * (size_t) (unsigned) mvr;
+        v.gr[0] = ld1 (gp);
+        v.gr[1] = ld1 (gp + 1);
+        v.gr[2] = ld1 (gp + 2);
     }
     if (ln_mse (MODE)) v.fv = ld1 (a.fimg + fidx);
     if (ln_hist (MODE) || MODE == LN_PZ_GRAD) v.fb = __ldg (a.fbin + fidx);
@@ -335,27 +339,23 @@ line_value (const Vox& v)
     return fmaf (v.w2[2], hi2 (cc) - lo2 (cc), lo2 (cc));
 }
 
-// dc/dv of one voxel (y weights wy) into the window of adjoint rows.
+// dc/dv of one voxel (y weights w) into the window of adjoint rows.
 template <int R>
 __device__ __forceinline__ void
-line_adjoint (const ulonglong2* __restrict__ wy, u64 cxy, float cz,
-    Row (&q)[4])
+line_adjoint (const u64* w, u64 cxy, float cz, Row (&q)[4])
 {
-    const ulonglong2 w01 = wy[0], w23 = wy[1];
-    q[R].xy = fma2 (w01.x, cxy, q[R].xy);
-    q[R].z = fmaf (lo2 (w01.x), cz, q[R].z);
-    q[(R + 1) & 3].xy = fma2 (w01.y, cxy, q[(R + 1) & 3].xy);
-    q[(R + 1) & 3].z = fmaf (lo2 (w01.y), cz, q[(R + 1) & 3].z);
-    q[(R + 2) & 3].xy = fma2 (w23.x, cxy, q[(R + 2) & 3].xy);
-    q[(R + 2) & 3].z = fmaf (lo2 (w23.x), cz, q[(R + 2) & 3].z);
-    q[(R + 3) & 3].xy = fma2 (w23.y, cxy, q[(R + 3) & 3].xy);
-    q[(R + 3) & 3].z = fmaf (lo2 (w23.y), cz, q[(R + 3) & 3].z);
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        Row& o = q[(R + b) & 3];
+        o.xy = fma2 (w[b], cxy, o.xy);
+        o.z = fmaf (lo2 (w[b]), cz, o.z);
+    }
 }
 
 // MSE at a loaded voxel and its adjoint.
 template <int MODE, int R>
 __device__ __forceinline__ void
-line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
+line_use (const LineArgs& a, int ly, const Vox& v,
     Row (&q)[4], float& scf, int& cnt)
 {
     float diff = line_value (v) - v.fv;
@@ -365,15 +365,15 @@ line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
     u64 cxy;
     float cz;
     if (MODE == LN_MSE_NEAREST) {
-        cxy = mul2 (pk (diff, diff), pk (v.gr.x, v.gr.y));
-        cz = diff * v.gr.z;
+        cxy = mul2 (pk (diff, diff), pk (v.gr[0], v.gr[1]));
+        cz = diff * v.gr[2];
     } else {
         float gd[3];
         trilinear_lerp_grad (a.g, v.w2, v.cr, gd);
         cxy = mul2 (pk (diff, diff), pk (gd[0], gd[1]));
         cz = diff * gd[2];
     }
-    line_adjoint<R> (wy, cxy, cz, q);
+    line_adjoint<R> (a.wy[ly], cxy, cz, q);
 }
 
 // Parzen pass 2 at a loaded voxel: 1/(N delta_m) * sum over the window's
@@ -384,8 +384,7 @@ line_use (const LineArgs& a, const ulonglong2* __restrict__ wy, const Vox& v,
 // -2s + 3s^2/2 (s = 1-f) and -f^2/2.
 template <bool AXIS, int R>
 __device__ __forceinline__ void
-line_use_pz (const LineArgs& a, const ulonglong2* __restrict__ wy,
-    const Vox& v, const float* slut, float scale, Row (&q)[4])
+line_use_pz (const LineArgs& a, int ly, const Vox& v, const float* slut, float scale, Row (&q)[4])
 {
     const float u = fmaf (line_value (v) - a.pz_min, a.pz_inv, 2.f);
     const int k0 = parzen_first_bin (u, a.bins);
@@ -403,7 +402,7 @@ line_use_pz (const LineArgs& a, const ulonglong2* __restrict__ wy,
         dc[c] = AXIS ? sc * (p[4 * c] * gi[c])
                      : sc * (p[c] * gi[0] + p[3 + c] * gi[1] + p[6 + c] * gi[2]);
     }
-    line_adjoint<R> (wy, pk (dc[0], dc[1]), dc[2], q);
+    line_adjoint<R> (a.wy[ly], pk (dc[0], dc[1]), dc[2], q);
 }
 
 // Histograms of a block: weights are summed as integers in 2^-24 units (no
@@ -555,7 +554,7 @@ line_kernel (const __grid_constant__ LineArgs a)
     const int vx = g.vpr[0], vy = g.vpr[1], vz = g.vpr[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int W = blockDim.x >> 5;
-    const LineSmem m = line_smem (vx, vy, vz, 0, 0);
+    const LineSmem m = line_smem (vx, vz, 0, 0);
 
     // the block: W warp columns (32 voxels along x in one plane) of tile
     // row tz, planes fastest, tiles ty0 .. along y
@@ -574,7 +573,6 @@ line_kernel (const __grid_constant__ LineArgs a)
     const int nj = nt + 3;
 
     u64* sbx = (u64*) (sm + m.bx);
-    u64* sby = (u64*) (sm + m.by);
     float* sbz = (float*) (sm + m.bz);
     ulonglong2* cz = (ulonglong2*) (sm + m.cz);
     // after the coefficients: the histograms (low and high halves of the
@@ -592,10 +590,6 @@ line_kernel (const __grid_constant__ LineArgs a)
     for (int o = threadIdx.x; o < 4 * vx; o += blockDim.x) {
         const float w = a.luts[o];
         sbx[o] = pk (w, w);
-    }
-    for (int o = threadIdx.x; o < 4 * vy; o += blockDim.x) {
-        const float w = a.luts[4 * vx + o];
-        sby[o] = pk (w, w);
     }
     for (int o = threadIdx.x; o < 4 * vz; o += blockDim.x) {
         sbz[o] = a.luts[4 * (vx + vy) + o];
@@ -687,7 +681,6 @@ line_kernel (const __grid_constant__ LineArgs a)
     // the fixed row index as a float, twice
     u64 jf2 = pk (i2f_small (g.roi_off[1] + ty0 * vy),
         i2f_small (g.roi_off[1] + ty0 * vy));
-    const ulonglong2* wy = (const ulonglong2*) sby;
     Run run;
     run.key = -1;
     int nvox = 0;
@@ -701,11 +694,11 @@ line_kernel (const __grid_constant__ LineArgs a)
         for (int ly = 0; ly < ny; ly++) {
             Vox v;
             line_load<MODE, AXIS, ROI, R> (a, col, g.roi_off[1] + y0 + ly,
-                jf2, wy + 2 * ly, p, v);
+                jf2, ly, p, v);
             if constexpr (ln_mse (MODE)) {
-                line_use<MODE, R> (a, wy + 2 * ly, v, q, scf, cnt);
+                line_use<MODE, R> (a, ly, v, q, scf, cnt);
             } else if constexpr (MODE == LN_PZ_GRAD) {
-                line_use_pz<AXIS, R> (a, wy + 2 * ly, v, slut, scale, q);
+                line_use_pz<AXIS, R> (a, ly, v, slut, scale, q);
             } else if constexpr (ln_hist (MODE)) {
                 if (MODE == LN_PZ_HIST) line_use_pz_hist (a, v, shist, run);
                 else line_use_mi_hist (a, v, shist, run);
@@ -1050,11 +1043,12 @@ line_finish_kernel (const __grid_constant__ LineFinishArgs a)
 bool
 line_plan (const BspGeom& g, LinePlan* p, int sm_count)
 {
+    static_assert (sizeof (p->wy) == 16 * LN_MAX_VPR, "y weights");
     // the regions that 10 mm grids give on 1 to 2.5 mm voxels, where it was
     // compared with the tile kernel (1.2 to 2.1 times as fast, 2^18 to 2^25
     // voxels); others stay there
     for (int d = 0; d < 3; d++) {
-        if (g.vpr[d] < 3 || g.vpr[d] > 10) return false;
+        if (g.vpr[d] < 3 || g.vpr[d] > LN_MAX_VPR) return false;
     }
     // corner offsets are 32-bit byte counts
     if ((long long) g.mdim[0] * g.mdim[1] * g.mdim[2] >= (1LL << 30)) return false;
@@ -1090,7 +1084,7 @@ line_plan (const BspGeom& g, LinePlan* p, int sm_count)
         const long long per_sm = (n + sm_count - 1) / sm_count;
         const double cost = (double) per_sm * (ty + LN_EDGE / g.vpr[1])
             / rate[std::min<long long> (per_sm, 4)];
-        const LineSmem m = line_smem (g.vpr[0], g.vpr[1], g.vpr[2], ty + 3, foot);
+        const LineSmem m = line_smem (g.vpr[0], g.vpr[2], ty + 3, foot);
         // (fewer than 65536 voxels a block: its histogram counters)
         if (p->ty && (m.total > 48 * 1024 || cost >= best
                 || p->nw * 32 * ty * g.vpr[1] > 65535)) continue;
@@ -1101,6 +1095,7 @@ line_plan (const BspGeom& g, LinePlan* p, int sm_count)
         p->smem = m.total;
     }
     p->threads = 32 * p->nw;
+    basis_lut (p->wy, g.vpr[1]);
     p->nblocks = p->gpr * p->nys * g.rdims[2];
     return p->nys < 65536 && g.rdims[2] < 65536 && p->smem <= 200 * 1024;
 }
@@ -1135,6 +1130,11 @@ line_args (const BspGeom& g, const LinePlan& p, const float* coeff,
         memcpy (&uy, &y, 4);
         return (u64) uy << 32 | ux;
     };
+    for (int v = 0; v < g.vpr[1]; v++) {
+        for (int k = 0; k < 4; k++) {
+            a.wy[v][k] = two (p.wy[4 * v + k], p.wy[4 * v + k]);
+        }
+    }
     a.step_y = two (0.f, g.fstep[4]);
     a.morg = two (g.morigin[0], g.morigin[1]);
     a.mprj = two (g.mproj[0], g.mproj[4]);
@@ -1152,7 +1152,7 @@ launch (const LinePlan& p, const LineArgs& a, cudaStream_t st)
     size_t smem = p.smem;
     if (ln_hist (MODE)) smem += (2 * a.bins * a.bins + a.bins) * sizeof (uint32_t);
     if (MODE == LN_PZ_GRAD) smem += a.bins * a.bins * sizeof (float);
-    if (smem > 48 * 1024) {
+    if (smem > LN_PLAIN_SMEM) {
         cudaError_t e = set_max_dynamic_smem ((const void*) k, (int) smem);
         if (e != cudaSuccess) return e;
     }
@@ -1178,7 +1178,7 @@ launch_mode (const LinePlan& p, const LineArgs& a, cudaStream_t st)
 
 cudaError_t
 launch_mse_line (const BspGeom& g, const LinePlan& p, int grad_mode,
-    const float* fimg, const float* mimg, const float4* mgrad4,
+    const float* fimg, const float* mimg, const float* mgrad,
     const float* coeff, const float* luts, float* rows, double* score_part,
     int* count_part, cudaStream_t st)
 {
@@ -1186,7 +1186,7 @@ launch_mse_line (const BspGeom& g, const LinePlan& p, int grad_mode,
     line_args (g, p, coeff, luts, a);
     a.fimg = fimg;
     a.mimg = mimg;
-    a.mgrad4 = mgrad4;
+    a.mgrad = mgrad;
     a.rows = rows;
     a.score_part = score_part;
     a.count_part = count_part;
@@ -1288,13 +1288,14 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     a.kxc = (g.cdims[0] + nbx - 1) / nbx;
     const int threads = (((a.kxc + 3) * g.vpr[0] + 2) / 2 + 31) / 32 * 32;
     // knots along z: a block reads 3 tile rows beyond its own, so few large
-    // blocks read less, but it takes some 400 to fill the chip; grids with
-    // fewer knots split a tile's planes over more threads
+    // blocks read less, but it takes some 300 to fill the chip (512x512x160:
+    // 36 us with 8, 44 with 4; 256x256x128: 13 with 4, 17 with 8); grids
+    // with fewer knots split a tile's planes over more threads
     a.kzc = 8;
     auto blocks = [&] () {
         return nbx * g.cdims[1] * ((g.cdims[2] + a.kzc - 1) / a.kzc);
     };
-    while (a.kzc > 2 && blocks () < 400) a.kzc /= 2;
+    while (a.kzc > 2 && blocks () < 300) a.kzc /= 2;
     int parts = 1;
     while (parts < 4 && parts < g.vpr[2] && threads * (parts + 1) <= 256
            && blocks () * threads * parts < 148 * 512) {
@@ -1308,7 +1309,7 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     auto k = line_finish_kernel<5>;
     if ((nz + rounds - 1) / rounds <= 3) k = line_finish_kernel<3>;
     else if ((nz + rounds - 1) / rounds == 4) k = line_finish_kernel<4>;
-    if (smem > 48 * 1024) {
+    if (smem > LN_PLAIN_SMEM) {
         cudaError_t e = set_max_dynamic_smem ((const void*) k, (int) smem);
         if (e != cudaSuccess) return e;
     }

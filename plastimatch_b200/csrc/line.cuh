@@ -18,6 +18,7 @@ struct LinePlan {
     int nblocks;
     int threads;
     size_t smem;
+    float wy[40];        // y basis table (vpr[1] * 4)
 };
 
 bool line_plan (const BspGeom& g, LinePlan* p, int sm_count);
@@ -30,7 +31,7 @@ line_row_elems (const BspGeom& g, const LinePlan& p)
 
 cudaError_t launch_mse_line (const BspGeom& g, const LinePlan& p,
     int grad_mode, const float* fimg, const float* mimg,
-    const float4* mgrad4, const float* coeff, const float* luts, float* rows,
+    const float* mgrad, const float* coeff, const float* luts, float* rows,
     double* score_part, int* count_part, cudaStream_t st);
 
 // Mattes MI: pass 1 (PVI-8 or Parzen histograms into hist, integer 2^-24

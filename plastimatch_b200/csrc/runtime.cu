@@ -229,10 +229,12 @@ inv3f (float* out, const float* m)
     return true;
 }
 
+namespace b200 {
+
 // Cubic B-spline basis table bx/by/bz_lut[vpr*4] as Bspline_xform::allocate
 // builds it (src/base/bspline_xform.cxx:73-99, 468-482): float argument,
 // double evaluation, rounded to float.
-static void
+void
 basis_lut (float* lut, int vpr)
 {
     for (int j = 0; j < 4; j++) {
@@ -249,6 +251,8 @@ basis_lut (float* lut, int vpr)
         }
     }
 }
+
+} // namespace b200
 
 // ------------------------------------------------------------- lifecycle --
 
@@ -936,7 +940,7 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
             c->d_count_part, c->stream));
     } else if (line_now (c)) {
         CK (launch_mse_line (g, c->lplan, c->opts.mse_grad, c->d_fixed,
-            c->d_moving, c->d_mgrad4, dcoeff, c->d_luts, c->d_rows,
+            c->d_moving, c->d_mgrad, dcoeff, c->d_luts, c->d_rows,
             c->d_score_part, c->d_count_part, c->stream));
     } else if (c->use_xl) {
         XlPlan plan = c->xplan;

@@ -33,6 +33,10 @@ CASES = [
     ((1040, 20, 12), (10, 6, 4), None, 0.0),       # two finish blocks along x
     ((48, 44, 36), (8, 9, 6), ((1, 0, 3), (47, 44, 33)), -15.0),
 ]
+# blocks whose dynamic shared memory lies just below 48 KB, where the static
+# arrays beside it need the larger limit
+LARGE_BLOCKS = [((224, 529, 28), (3, 3, 9), None, 0.0),
+                ((81, 439, 106), (4, 3, 10), None, 0.0)]
 
 
 def _volume(dim, seed, dcos, origin=(0.0, 0.0, 0.0)):
@@ -54,7 +58,7 @@ def _case(dim, vpr, roi, angle, seed=71):
 
 
 @pytest.mark.parametrize("grad", ["nearest", "trilinear"])
-@pytest.mark.parametrize("case", CASES)
+@pytest.mark.parametrize("case", CASES + LARGE_BLOCKS)
 def test_line_kernel_matches_tile_kernel(case, grad):
     fixed, moving, grid, coeff = _case(*case)
     out = []
