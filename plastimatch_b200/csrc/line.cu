@@ -98,6 +98,7 @@ struct LineArgs {
     float pz_min, pz_inv;                   // moving value -> window centre
     float* out;          // field (xyz per voxel) or warped image
     float outside;
+    bool roi_same;       // the moving ROI is a mask on the moving image's grid
     int ty, j, nxs;
     // y weights of each row of a tile, each twice; in the parameter bank,
     // since they are the same for every thread: shared memory would return
@@ -202,6 +203,7 @@ struct Vox {
     float w2[3];
     uint32_t mq[2];
     int fb, fidx, clamp;
+    int roi;             // moving ROI's mask at the position
     bool ok;
 };
 
@@ -263,7 +265,7 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
     }
     jf2 = add2 (jf2, pk (1.f, 1.f));
     bool in = col.live;
-    int bits[3];
+    int bits[3], rbits[3];
     v.clamp = 0;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -271,8 +273,9 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
         // li_clamp without conversions (see locate_nx): floor in the low
         // mantissa bits of max(ma, 0) + 2^23 rounded down, corner at
         // most dim - 2, fraction saturated to [0, 1]
-        bits[d] = min (__float_as_int (__fadd_rd (fmaxf (ma[d], 0.f),
-            8388608.f)), a.mtop[d]);
+        bits[d] = __float_as_int (__fadd_rd (fmaxf (ma[d], 0.f), 8388608.f));
+        if (ROI) rbits[d] = min (bits[d], a.mtop[d] + 1);
+        bits[d] = min (bits[d], a.mtop[d]);
         v.w2[d] = __saturatef (ma[d] - (__int_as_float (bits[d]) - 8388608.f));
         if (MODE == LN_PZ_GRAD && (ma[d] < 0.f || ma[d] >= g.m_fmax[d] + 1.f)) {
             v.clamp |= 1 << d;
@@ -288,12 +291,19 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
         v.cr[2] = dz;
         return;
     }
-    if (ROI) {
-        const float dd[3] = {lo2 (dxy), hi2 (dxy), dz};
-        in = in && roi_fixed_ok (g, fidx);
-        if (in) in = roi_moving_ok (g, fx, dd);
-    }
     v.ok = in;
+    if (ROI) {
+        // the moving mask's byte goes out with the other loads; where the
+        // mask lies on the moving image's own grid its index is the clamped
+        // floor of the position (the same operations as inside_roi)
+        if (AXIS && a.roi_same) {
+            v.roi = __ldg (g.mroi + (rbits[0] + g.mdim[0] * (rbits[1]
+                + g.mdim[1] * rbits[2]) + a.midx0));
+        } else {
+            const float dd[3] = {lo2 (dxy), hi2 (dxy), dz};
+            v.roi = roi_moving_ok (g, fx, dd);
+        }
+    }
     const int dx = g.mdim[0], dxym = g.mdim[0] * g.mdim[1];
     const unsigned off = (unsigned) mvf * 4u;
     const char* b0 = (const char*) a.mimg;
@@ -691,10 +701,28 @@ line_kernel (const __grid_constant__ LineArgs a)
         const int ny = min (vy, g.roi_dim[1] - y0);
         float scf = 0.f;
         int cnt = 0;
+        // the column's fixed mask over the tile, a bit a row; rows that no
+        // lane of the warp has inside are skipped
+        unsigned inside = ~0u, any = ~0u;
+        if (ROI && g.fmask) {
+            inside = 0u;
+            const uint8_t* fm = g.fmask + col.frow + (g.roi_off[1] + y0) * g.fdim[0];
+#pragma unroll 5
+            for (int ly = 0; ly < ny; ly++) {
+                inside |= (unsigned) (__ldg (fm + ly * g.fdim[0]) & 1) << ly;
+            }
+            any = __reduce_or_sync (0xffffffffu, inside);
+        }
         for (int ly = 0; ly < ny; ly++) {
             Vox v;
+            if (ROI) {
+                if (!(any >> ly & 1u)) continue;
+                const float f = i2f_small (g.roi_off[1] + y0 + ly);
+                jf2 = pk (f, f);
+            }
             line_load<MODE, AXIS, ROI, R> (a, col, g.roi_off[1] + y0 + ly,
                 jf2, ly, p, v);
+            if (ROI) v.ok = v.ok && v.roi && (inside >> ly & 1u);
             if constexpr (ln_mse (MODE)) {
                 line_use<MODE, R> (a, ly, v, q, scf, cnt);
             } else if constexpr (MODE == LN_PZ_GRAD) {
@@ -1134,6 +1162,14 @@ line_args (const BspGeom& g, const LinePlan& p, const float* coeff,
         for (int k = 0; k < 4; k++) {
             a.wy[v][k] = two (p.wy[4 * v + k], p.wy[4 * v + k]);
         }
+    }
+    a.roi_same = g.mroi != nullptr;
+    for (int d = 0; d < 3; d++) {
+        a.roi_same = a.roi_same && g.mroi_dim[d] == g.mdim[d]
+            && g.mroi_origin[d] == g.morigin[d];
+    }
+    for (int i = 0; i < 9; i++) {
+        a.roi_same = a.roi_same && g.mroi_proj[i] == g.mproj[i];
     }
     a.step_y = two (0.f, g.fstep[4]);
     a.morg = two (g.morigin[0], g.morigin[1]);
