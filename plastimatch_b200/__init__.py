@@ -435,7 +435,7 @@ class Context:
                                            _ptr(score_out), _ptr(grad_out),
                                            _ptr(nvox_out)), self._h)
             return score_out, grad_out, nvox_out
-        g = np.zeros(self.num_coeff, np.float32)
+        g = np.empty(self.num_coeff, np.float32)
         s = C.c_float()
         n = C.c_int64()
         _check(lib().b200bsp_score_mse(self._h, _ptr(coeff), C.addressof(s),
@@ -470,7 +470,7 @@ class Context:
 
     def score_mi(self, coeff, with_hist=False):
         b = None
-        g = np.zeros(self.num_coeff, np.float32)
+        g = np.empty(self.num_coeff, np.float32)
         s = C.c_float()
         n = C.c_int64()
         fh = mh = jh = None
@@ -561,7 +561,7 @@ class Context:
 
     def score(self, coeff, metric="mse", lam=1.0, reg: RegParms | None = None):
         """bspline_score(): (total_score, total_grad, smetric, num_vox)."""
-        g = np.zeros(self.num_coeff, np.float32)
+        g = np.empty(self.num_coeff, np.float32)
         ts, sm = C.c_float(), C.c_float()
         n = C.c_int64()
         _check(lib().b200bsp_score(self._h, _ptr(coeff),

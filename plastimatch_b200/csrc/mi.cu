@@ -242,63 +242,35 @@ eqsp_range (const float* d_img, size_t n, int bins, float* d_scratch,
     return B200BSP_OK;
 }
 
-int
-mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist)
+void
+mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
+    bool line, Arena& dev, Arena& pinned)
 {
     s->bins = bins;
     s->window = window;
     s->hist = hist;
-    if (hist == B200BSP_MI_HIST_VOPT
-        && (cudaMalloc (&s->d_fkey, MI_VOPT_KEYS * sizeof (int)) != cudaSuccess
-            || cudaMalloc (&s->d_mkey, MI_VOPT_KEYS * sizeof (int)) != cudaSuccess)) {
-        cudaGetLastError ();
-        return B200BSP_E_OOM;
-    }
-    size_t nf = (size_t) g.fdim[0] * g.fdim[1] * g.fdim[2];
-    size_t nm = (size_t) g.mdim[0] * g.mdim[1] * g.mdim[2];
-    size_t nh = 2 * bins + bins * bins + 1;
-    if (cudaMalloc (&s->d_fbin, nf) != cudaSuccess
-        || cudaMalloc (&s->d_mbin, nm) != cudaSuccess
-        || cudaMalloc (&s->d_hist, nh * sizeof (unsigned long long)) != cudaSuccess
-        || cudaMalloc (&s->d_histd, nh * sizeof (double)) != cudaSuccess
-        || cudaMalloc (&s->d_lut, bins * bins * sizeof (float)) != cudaSuccess
-        || cudaMalloc (&s->d_nvf, 2 * sizeof (float)) != cudaSuccess
-        || cudaMalloc (&s->d_minmax, 2 * 296 * sizeof (float)) != cudaSuccess
-        || cudaMalloc (&s->d_part, (size_t) 64 * 3 * g.ntiles * sizeof (float))
-            != cudaSuccess
-        || cudaMalloc (&s->d_score_part, g.ntiles * sizeof (double)) != cudaSuccess
-        || cudaMalloc (&s->d_count_part, g.ntiles * sizeof (int)) != cudaSuccess
-        || cudaMallocHost (&s->h_histd, nh * sizeof (double)) != cudaSuccess
-        || cudaMallocHost (&s->h_res, sizeof (DevResult)) != cudaSuccess) {
-        cudaGetLastError ();
-        return B200BSP_E_OOM;
-    }
-    return B200BSP_OK;
-}
-
-int
-mi_alloc_line (MiState* s, const BspGeom& g)
-{
+    const size_t nf = (size_t) g.fdim[0] * g.fdim[1] * g.fdim[2];
     const size_t nm = (size_t) g.mdim[0] * g.mdim[1] * g.mdim[2];
-    if (s->window != B200BSP_MI_PVI8) return B200BSP_OK;
-    if (cudaMalloc (&s->d_mquad, nm * sizeof (uint32_t)) != cudaSuccess) {
-        cudaGetLastError ();
-        return B200BSP_E_OOM;
+    const size_t nh = 2 * bins + bins * bins + 1;
+    if (hist == B200BSP_MI_HIST_VOPT) {
+        dev.add (&s->d_fkey, MI_VOPT_KEYS * sizeof (int));
+        dev.add (&s->d_mkey, MI_VOPT_KEYS * sizeof (int));
     }
-    return B200BSP_OK;
-}
-
-void
-mi_free (MiState* s)
-{
-    cudaFree (s->d_fbin); cudaFree (s->d_mbin); cudaFree (s->d_hist);
-    cudaFree (s->d_histd); cudaFree (s->d_lut); cudaFree (s->d_nvf);
-    cudaFree (s->d_minmax); cudaFree (s->d_part); cudaFree (s->d_score_part);
-    cudaFree (s->d_count_part);
-    cudaFree (s->d_fkey); cudaFree (s->d_mkey);
-    cudaFree (s->d_mquad);
-    cudaFreeHost (s->h_histd); cudaFreeHost (s->h_res);
-    *s = MiState ();
+    dev.add (&s->d_fbin, nf);
+    dev.add (&s->d_mbin, nm);
+    if (line && window == B200BSP_MI_PVI8) {
+        dev.add (&s->d_mquad, nm * sizeof (uint32_t));
+    }
+    dev.add (&s->d_hist, nh * sizeof (unsigned long long));
+    dev.add (&s->d_histd, nh * sizeof (double));
+    dev.add (&s->d_lut, bins * bins * sizeof (float));
+    dev.add (&s->d_nvf, 2 * sizeof (float));
+    dev.add (&s->d_minmax, 2 * 296 * sizeof (float));
+    dev.add (&s->d_part, (size_t) 64 * 3 * g.ntiles * sizeof (float));
+    dev.add (&s->d_score_part, g.ntiles * sizeof (double));
+    dev.add (&s->d_count_part, g.ntiles * sizeof (int));
+    pinned.add (&s->h_histd, nh * sizeof (double));
+    pinned.add (&s->h_res, sizeof (DevResult));
 }
 
 int

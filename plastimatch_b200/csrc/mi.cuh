@@ -49,11 +49,9 @@ struct MiState {
     DevResult* h_res = nullptr;
 };
 
-int mi_alloc (MiState* s, const BspGeom& g, int bins, int window,
-    int hist = 0);
-// The line kernel's bin image (contexts that may run it).
-int mi_alloc_line (MiState* s, const BspGeom& g);
-void mi_free (MiState* s);
+// Asks for the state's buffers (line: for the line kernel as well).
+void mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
+    bool line, Arena& dev, Arena& pinned);
 int mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
     const float* d_moving, size_t nf, size_t nm, cudaStream_t st);
 // passes: MI_PASS_HIST (histograms into d_hist), MI_PASS_GRAD (score and

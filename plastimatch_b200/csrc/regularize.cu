@@ -374,8 +374,25 @@ reg_pass_z (RegPlan plan, int cx, int cy, int cz, int nk,
 
 // ---- host -------------------------------------------------------------------
 
+void
+reg_alloc (RegState* s, const BspGeom& g, Arena& dev, Arena& pinned)
+{
+    const int cx = g.cdims[0], cy = g.cdims[1], cz = g.cdims[2];
+    // pass z's grid: 32 knots along x x one y row x REG_TY planes
+    s->nblocks = ((cx + 31) / 32) * cy * ((cz + REG_TY - 1) / REG_TY);
+    dev.add (&s->d_gx, sizeof (double) * 6 * cx * 7);
+    dev.add (&s->d_gy, sizeof (double) * 6 * cy * 7);
+    dev.add (&s->d_hz, sizeof (double) * REG_E_MAX * cz * 7);
+    dev.add (&s->d_t1, sizeof (double) * REG_T1_MAX * (size_t) g.nknots);
+    dev.add (&s->d_t2, sizeof (double) * REG_T2_MAX * (size_t) g.nknots);
+    dev.add (&s->d_part, sizeof (double) * s->nblocks);
+    dev.add (&s->d_arrive, sizeof (unsigned));
+    dev.add (&s->d_score, sizeof (double));
+    pinned.add (&s->h_score, sizeof (double));
+}
+
 int
-reg_alloc (RegState* s, const BspGeom& g, const float grid_spac[3])
+reg_init (RegState* s, const BspGeom& g, const float grid_spac[3])
 {
     for (int d = 0; d < 3; d++) {
         s->cdims[d] = g.cdims[d];
@@ -389,28 +406,11 @@ reg_alloc (RegState* s, const BspGeom& g, const float grid_spac[3])
             (int) (REG_T1_MAX * slot)) != cudaSuccess
         || set_max_dynamic_smem ((const void*) reg_pass_z,
             (int) (REG_T2_MAX * slot + REG_E_MAX * REG_TY * 7 * sizeof (double)))
-            != cudaSuccess) {
+            != cudaSuccess
+        || cudaMemset (s->d_arrive, 0, sizeof (unsigned)) != cudaSuccess) {
         return B200BSP_E_CUDA;
     }
-    // pass z's grid: 32 knots along x x one y row x REG_TY planes
-    s->nblocks = ((g.cdims[0] + 31) / 32) * g.cdims[1]
-        * ((g.cdims[2] + REG_TY - 1) / REG_TY);
     const int cx = g.cdims[0], cy = g.cdims[1], cz = g.cdims[2];
-    if (cudaMalloc (&s->d_gx, sizeof (double) * 6 * cx * 7) != cudaSuccess
-        || cudaMalloc (&s->d_gy, sizeof (double) * 6 * cy * 7) != cudaSuccess
-        || cudaMalloc (&s->d_hz, sizeof (double) * REG_E_MAX * cz * 7) != cudaSuccess
-        || cudaMalloc (&s->d_t1, sizeof (double) * REG_T1_MAX * (size_t) g.nknots)
-            != cudaSuccess
-        || cudaMalloc (&s->d_t2, sizeof (double) * REG_T2_MAX * (size_t) g.nknots)
-            != cudaSuccess
-        || cudaMalloc (&s->d_part, sizeof (double) * s->nblocks) != cudaSuccess
-        || cudaMalloc (&s->d_arrive, sizeof (unsigned)) != cudaSuccess
-        || cudaMemset (s->d_arrive, 0, sizeof (unsigned)) != cudaSuccess
-        || cudaMalloc (&s->d_score, sizeof (double)) != cudaSuccess
-        || cudaMallocHost (&s->h_score, sizeof (double)) != cudaSuccess) {
-        cudaGetLastError ();
-        return B200BSP_E_OOM;
-    }
     // Unweighted knot-axis bands for the six factor kinds.  Knot x takes
     // the Z factor (grid spacing 2), knot y the Y factor (spacing 1), knot
     // z the X factor (spacing 0).
@@ -438,16 +438,6 @@ reg_alloc (RegState* s, const BspGeom& g, const float grid_spac[3])
         return B200BSP_E_CUDA;
     }
     return B200BSP_OK;
-}
-
-void
-reg_free (RegState* s)
-{
-    cudaFree (s->d_gx); cudaFree (s->d_gy); cudaFree (s->d_hz);
-    cudaFree (s->d_t1); cudaFree (s->d_t2); cudaFree (s->d_part);
-    cudaFree (s->d_arrive);
-    cudaFree (s->d_score); cudaFreeHost (s->h_score);
-    *s = RegState ();
 }
 
 // Build the pass plan and the weighted z bands for one set of weights.

@@ -6,6 +6,7 @@
 
 #include "../../include/plastimatch_b200.h"
 #include "bsp_common.cuh"
+#include "kernels.cuh"
 
 namespace b200 {
 
@@ -48,8 +49,9 @@ struct RegState {
     std::vector<double> gz_host;    // [6][cdims2][7] unweighted z bands
 };
 
-int reg_alloc (RegState* s, const BspGeom& g, const float grid_spac[3]);
-void reg_free (RegState* s);
+// Asks for the state's buffers; reg_init fills them once they are there.
+void reg_alloc (RegState* s, const BspGeom& g, Arena& dev, Arena& pinned);
+int reg_init (RegState* s, const BspGeom& g, const float grid_spac[3]);
 // d_grad: the gradient is added into it (float, one double rounding per
 // entry); d_grad64 (instead): stored there in double.  The score goes to
 // s->d_score (double).

@@ -43,6 +43,9 @@ struct b200bsp_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;
 
+    // every buffer of the context that is there from its creation on
+    void* d_slab = nullptr;
+    void* h_slab = nullptr;
     float* d_fixed = nullptr;
     float* d_moving = nullptr;
     float* d_mgrad = nullptr;
@@ -61,7 +64,12 @@ struct b200bsp_ctx {
     float* d_inv_dc = nullptr;
     DevResult* h_res = nullptr;
     DevResult* h_res_dev = nullptr;   // device alias of h_res (mapped)
-    float* h_scalar = nullptr;
+    float* h_scalar = nullptr;        // page-locked: [0] scores, [8] error flag
+    // page-locked staging of host coefficients and gradients, for calls that
+    // wait for their results; events of the gradient's parts
+    float* h_up = nullptr;
+    float* h_down = nullptr;
+    cudaEvent_t ev_down[4] = {nullptr, nullptr, nullptr, nullptr};
 
     PartLayout lay;
     TcPlan plan;
@@ -296,28 +304,20 @@ check_volume (const b200bsp_volume* v, const char* what)
 static void
 free_all (b200bsp_ctx* c)
 {
-    cudaFree (c->d_fixed); cudaFree (c->d_moving); cudaFree (c->d_mgrad);
+    cudaFree (c->d_slab);
+    cudaFreeHost (c->h_slab);
     cudaFree (c->d_out);
-    cudaFree (c->d_mgrad4);
-    cudaFree (c->d_rows);
     if (c->ev_fork) cudaEventDestroy (c->ev_fork);
     if (c->ev_join) cudaEventDestroy (c->ev_join);
     if (c->aux_stream) cudaStreamDestroy (c->aux_stream);
-    cudaFree (c->d_coeff); cudaFree (c->d_luts); cudaFree (c->d_grad);
-    cudaFree (c->d_grad64); cudaFree (c->d_part); cudaFree (c->d_score_part);
-    cudaFree (c->d_count_part); cudaFree (c->d_res); cudaFree (c->d_err);
-    cudaFree (c->d_qlut); cudaFree (c->d_xtab); cudaFree (c->d_inv_dc);
+    cudaFree (c->d_qlut); cudaFree (c->d_xtab);
     cudaFree (c->d_lm_p); cudaFree (c->d_lm_w); cudaFree (c->d_lm_fm);
     cudaFree (c->d_lm_dc);
     cudaFree (c->d_fmask); cudaFree (c->d_mroi);
-    cudaFreeHost (c->h_res); cudaFreeHost (c->h_scalar);
-    mi_free (&c->mi);
-    reg_free (&c->reg);
     if (c->opt_ws_free) c->opt_ws_free (c->opt_ws);
     c->opt_ws = nullptr;
     for (auto& e : c->ev) if (e) cudaEventDestroy (e);
-    cudaFree (c->d_reg_grad64);
-    cudaFree (c->d_total);
+    for (auto& e : c->ev_down) if (e) cudaEventDestroy (e);
     if (c->own_stream) cudaStreamDestroy (c->own_stream);
 }
 
@@ -570,6 +570,7 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
     size_t nf = (size_t) g.fdim[0] * g.fdim[1] * g.fdim[2];
     size_t nm = (size_t) g.mdim[0] * g.mdim[1] * g.mdim[2];
     int rc2 = B200BSP_OK;
+    Arena dev, pinned;
     auto alloc = [&](void** p, size_t bytes) {
         if (rc2) return;
         if (g_fail_alloc > 0 && --g_fail_alloc == 0) {
@@ -577,12 +578,7 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
                 bytes);
             return;
         }
-        cudaError_t e = cudaMalloc (p, bytes);
-        if (e != cudaSuccess) {
-            cudaGetLastError ();
-            rc2 = fail (c, B200BSP_E_OOM, "cudaMalloc(%zu): %s", bytes,
-                cudaGetErrorString (e));
-        }
+        dev.add ((void**) p, bytes);
     };
     alloc ((void**) &c->d_fixed, nf * sizeof (float));
     alloc ((void**) &c->d_moving, nm * sizeof (float));
@@ -626,16 +622,10 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
     alloc ((void**) &c->d_inv_dc, 9 * sizeof (float));
     int nlut = 4 * (g.vpr[0] + g.vpr[1] + g.vpr[2]);
     alloc ((void**) &c->d_luts, nlut * sizeof (float));
-    if (!rc2 && (cudaMallocHost ((void**) &c->h_res, sizeof (DevResult)) != cudaSuccess
-        || cudaMallocHost ((void**) &c->h_scalar, 64) != cudaSuccess)) {
-        cudaGetLastError ();
-        rc2 = fail (c, B200BSP_E_OOM, "cudaMallocHost failed");
-    }
-    if (!rc2 && cudaHostGetDevicePointer ((void**) &c->h_res_dev, c->h_res, 0)
-        != cudaSuccess) {
-        cudaGetLastError ();
-        c->h_res_dev = nullptr;          // result block then comes by copy
-    }
+    pinned.add (&c->h_res, sizeof (DevResult));
+    pinned.add (&c->h_scalar, 64);
+    pinned.add (&c->h_up, c->num_coeff * sizeof (float));
+    pinned.add (&c->h_down, c->num_coeff * sizeof (float));
 
     // Tile partial-gradient layout of the chosen form.
     size_t part_elems = 0;
@@ -690,16 +680,27 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
     score_parts = std::max (score_parts, (size_t) std::max (c->nscore_parts, 1));
     alloc ((void**) &c->d_score_part, score_parts * sizeof (double));
     alloc ((void**) &c->d_count_part, score_parts * sizeof (int));
+    mi_alloc (&c->mi, c->geom, o.mi_bins, o.mi_window, o.mi_hist, c->use_line,
+        dev, pinned);
+    reg_alloc (&c->reg, c->geom, dev, pinned);
+    if (!rc2) {
+        cudaError_t e = dev.take (false, &c->d_slab);
+        if (e == cudaSuccess) e = pinned.take (true, &c->h_slab);
+        if (e != cudaSuccess) {
+            cudaGetLastError ();
+            rc2 = fail (c, B200BSP_E_OOM, "%zu bytes of device and %zu of "
+                "page-locked memory: %s", dev.bytes (), pinned.bytes (),
+                cudaGetErrorString (e));
+        }
+    }
+    if (!rc2 && cudaHostGetDevicePointer ((void**) &c->h_res_dev, c->h_res, 0)
+        != cudaSuccess) {
+        cudaGetLastError ();
+        c->h_res_dev = nullptr;          // result block then comes by copy
+    }
     if (!rc2 && o.form == B200BSP_FORM_TC) {
         rc2 = tc_build_tables (c->geom, c->plan, &c->d_qlut);
         if (rc2) rc2 = fail (c, rc2, "tensor-core tables: %s", cudaGetErrorString (cudaGetLastError ()));
-    }
-    if (!rc2 && mi_alloc (&c->mi, c->geom, o.mi_bins, o.mi_window,
-            o.mi_hist)) {
-        rc2 = fail (c, B200BSP_E_OOM, "MI buffers: out of device memory");
-    }
-    if (!rc2 && c->use_line && mi_alloc_line (&c->mi, c->geom)) {
-        rc2 = fail (c, B200BSP_E_OOM, "MI buffers: out of device memory");
     }
     if (!rc2) {
         // Bspline_xform::grid_spac = vox_per_rgn * |spacing| (float)
@@ -707,7 +708,7 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
         for (int d = 0; d < 3; d++) {
             gsp[d] = (float) g.vpr[d] * std::fabs (c->fixed.spacing[d]);
         }
-        if (reg_alloc (&c->reg, c->geom, gsp)) {
+        if (reg_init (&c->reg, c->geom, gsp)) {
             rc2 = fail (c, B200BSP_E_OOM, "regulariser buffers");
         }
     }
@@ -725,6 +726,14 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
         || cudaEventCreateWithFlags (&c->ev_fork, cudaEventDisableTiming)
         != cudaSuccess
         || cudaEventCreateWithFlags (&c->ev_join, cudaEventDisableTiming)
+        != cudaSuccess
+        || cudaEventCreateWithFlags (&c->ev_down[0], cudaEventDisableTiming)
+        != cudaSuccess
+        || cudaEventCreateWithFlags (&c->ev_down[1], cudaEventDisableTiming)
+        != cudaSuccess
+        || cudaEventCreateWithFlags (&c->ev_down[2], cudaEventDisableTiming)
+        != cudaSuccess
+        || cudaEventCreateWithFlags (&c->ev_down[3], cudaEventDisableTiming)
         != cudaSuccess) {
         cudaGetLastError ();
         free_all (c);
@@ -873,8 +882,53 @@ struct OutPtrs {
     long long* nvox;
 };
 
+// Host coefficients through the page-locked staging buffer, in parts: the
+// copy into it overlaps the transfer of the part before (1 MB: 50 us, 83 as
+// one pageable copy).  Only for calls that wait for their results, so that
+// the buffer is free again when they return.
+constexpr int64_t STAGE_PART = 64 * 1024;          // floats
+
+static cudaError_t
+stage_up (b200bsp_ctx* c, const float* coeff)
+{
+    for (int64_t o = 0; o < c->num_coeff; o += STAGE_PART) {
+        const size_t n = std::min (STAGE_PART, c->num_coeff - o);
+        memcpy (c->h_up + o, coeff + o, n * sizeof (float));
+        const cudaError_t e = cudaMemcpyAsync (c->d_coeff + o, c->h_up + o,
+            n * sizeof (float), cudaMemcpyHostToDevice, c->stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// The gradient in d_grad to host memory the same way, after everything else
+// on the stream (up to four parts, each waited for and copied out while the
+// next one is on its way); returns when the last one is there.
+static cudaError_t
+stage_down (b200bsp_ctx* c, float* grad)
+{
+    const int64_t part = std::max<int64_t> (STAGE_PART, (c->num_coeff + 3) / 4);
+    cudaError_t e = cudaSuccess;
+    int k = 0;
+    for (int64_t o = 0; o < c->num_coeff && e == cudaSuccess; o += part, k++) {
+        const size_t n = std::min (part, c->num_coeff - o);
+        e = cudaMemcpyAsync (c->h_down + o, c->d_grad + o, n * sizeof (float),
+            cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess) e = cudaEventRecord (c->ev_down[k], c->stream);
+    }
+    k = 0;
+    for (int64_t o = 0; o < c->num_coeff && e == cudaSuccess; o += part, k++) {
+        const size_t n = std::min (part, c->num_coeff - o);
+        e = cudaEventSynchronize (c->ev_down[k]);
+        if (e == cudaSuccess) memcpy (grad + o, c->h_down + o, n * sizeof (float));
+    }
+    return e;
+}
+
+// waits: the call returns only when its results are there.
 static int
-begin_eval (b200bsp_ctx* c, const float* coeff, const float** dcoeff)
+begin_eval (b200bsp_ctx* c, const float* coeff, const float** dcoeff,
+    bool waits = false)
 {
     if (!c) return B200BSP_E_BADARG;
     if (!c->images_set) return fail (c, B200BSP_E_STATE, "images not set");
@@ -883,8 +937,13 @@ begin_eval (b200bsp_ctx* c, const float* coeff, const float** dcoeff)
     if (is_device_ptr (coeff)) {
         *dcoeff = coeff;
     } else {
-        CK (cudaMemcpyAsync (c->d_coeff, coeff, c->num_coeff * sizeof (float),
-            cudaMemcpyHostToDevice, c->stream));
+        if (waits && !mapped_alias ((void*) coeff)) {
+            CK (stage_up (c, coeff));
+        } else {
+            CK (cudaMemcpyAsync (c->d_coeff, coeff,
+                c->num_coeff * sizeof (float), cudaMemcpyHostToDevice,
+                c->stream));
+        }
         *dcoeff = c->d_coeff;
     }
     if (c->timing) {
@@ -1011,11 +1070,11 @@ b200bsp_score_mse (b200bsp_ctx* c, const float* coeff, float* score,
     float* grad, int64_t* num_vox)
 {
     const float* dcoeff = nullptr;
-    int rc = begin_eval (c, coeff, &dcoeff);
+    const bool dev_out = is_device_ptr (grad) && (!score || is_device_ptr (score))
+        && (!num_vox || is_device_ptr (num_vox)) && is_device_ptr (coeff);
+    int rc = begin_eval (c, coeff, &dcoeff, !dev_out);
     if (rc) return rc;
-    bool dev_out = is_device_ptr (grad) && (!score || is_device_ptr (score))
-        && (!num_vox || is_device_ptr (num_vox));
-    if (dev_out && is_device_ptr (coeff)) {
+    if (dev_out) {
         rc = run_mse (c, dcoeff, grad, nullptr, score, nullptr,
             (long long*) num_vox);
         if (rc) return rc;
@@ -1033,10 +1092,7 @@ b200bsp_score_mse (b200bsp_ctx* c, const float* coeff, float* score,
         CK (cudaMemcpyAsync (c->h_res, c->d_res, sizeof (DevResult),
             cudaMemcpyDeviceToHost, c->stream));
     }
-    if (grad && g_dev == c->d_grad) {
-        CK (cudaMemcpyAsync (grad, c->d_grad, c->num_coeff * sizeof (float),
-            cudaMemcpyDeviceToHost, c->stream));
-    }
+    if (grad && g_dev == c->d_grad) CK (stage_down (c, grad));
     rc = end_eval (c, true);
     if (rc) return rc;
     if (score) *score = c->h_res->score_f;
@@ -1286,7 +1342,7 @@ b200bsp_score_mi (b200bsp_ctx* c, const float* coeff, float* score,
             "cover the fixed image");
     }
     const float* dcoeff = nullptr;
-    int rc = begin_eval (c, coeff, &dcoeff);
+    int rc = begin_eval (c, coeff, &dcoeff, true);
     if (rc) return rc;
     float* g_dev = is_device_ptr (grad) ? grad : c->d_grad;
     rc = mi_passes (c, dcoeff, g_dev, nullptr, MI_PASS_HIST | MI_PASS_GRAD);
@@ -1296,16 +1352,16 @@ b200bsp_score_mi (b200bsp_ctx* c, const float* coeff, float* score,
     MiResult mr;
     rc = mi_fetch (&c->mi, c->d_res, f_hist, m_hist, j_hist, c->stream);
     if (rc) return fail (c, rc, "MI fetch failed");
-    if (grad && g_dev == c->d_grad) {
-        CK (cudaMemcpyAsync (grad, c->d_grad, c->num_coeff * sizeof (float),
-            cudaMemcpyDeviceToHost, c->stream));
-    }
+    int* err = (int*) (c->h_scalar + 8);
+    CK (cudaMemcpyAsync (err, c->d_err, sizeof (int), cudaMemcpyDeviceToHost,
+        c->stream));
+    if (grad && g_dev == c->d_grad) CK (stage_down (c, grad));
     rc = end_eval (c, true);
     if (rc) return rc;
     mi_finish (&c->mi, &mr);
     if (score) *score = mr.score_f;
     if (num_vox) *num_vox = mr.num_vox;
-    return check_device_error (c);
+    return check_device_error (c, *err);
 }
 
 extern "C" int
@@ -1689,10 +1745,11 @@ b200bsp_landmarks_score (b200bsp_ctx* c, const float* coeff, float* lmetric,
 static int
 score_mse_device (b200bsp_ctx* c, const float* coeff, float lambda,
     const b200bsp_reg_parms* reg, float* total_score, float* total_grad,
-    float* smetric, int64_t* num_vox)
+    float* smetric, int64_t* num_vox, DevResult* res_host = nullptr,
+    bool waits = false)
 {
     const float* dcoeff = nullptr;
-    int rc = begin_eval (c, coeff, &dcoeff);
+    int rc = begin_eval (c, coeff, &dcoeff, waits);
     if (rc) return rc;
     FinishCombine cb;
     cb.lambda = lambda;
@@ -1709,7 +1766,7 @@ score_mse_device (b200bsp_ctx* c, const float* coeff, float lambda,
         }
     }
     rc = run_mse (c, dcoeff, total_grad, nullptr, smetric, nullptr,
-        (long long*) num_vox, nullptr, cb, reg ? c->ev_join : nullptr,
+        (long long*) num_vox, res_host, cb, reg ? c->ev_join : nullptr,
         [&] () {
             // between the MSE kernel's launch and the finish kernel's
             if (!reg) return B200BSP_OK;
@@ -1722,7 +1779,7 @@ score_mse_device (b200bsp_ctx* c, const float* coeff, float lambda,
             return B200BSP_OK;
         });
     c->tc_grid = grid0;
-    if (rc) return rc;
+    if (rc || waits) return rc;
     return end_eval (c, false);
 }
 
@@ -1734,7 +1791,8 @@ __global__ void
 mi_combine_kernel (const DevResult* __restrict__ res, float lambda,
     const double* __restrict__ reg_grad, const double* __restrict__ reg_score,
     float* __restrict__ grad, long long n, float* __restrict__ total,
-    float* __restrict__ smetric, long long* __restrict__ nvox)
+    float* __restrict__ smetric, long long* __restrict__ nvox,
+    const int* __restrict__ err, DevResult* __restrict__ res_host)
 {
     for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x;
          i < n; i += (long long) gridDim.x * blockDim.x) {
@@ -1748,6 +1806,11 @@ mi_combine_kernel (const DevResult* __restrict__ res, float lambda,
         *total = tot;
         if (smetric) *smetric = res->score_f;
         if (nvox) *nvox = res->num_vox;
+        if (res_host) {
+            DevResult r = *res;
+            r.error = *err;
+            *res_host = r;
+        }
     }
 }
 
@@ -1757,7 +1820,8 @@ mi_combine_kernel (const DevResult* __restrict__ res, float lambda,
 static int
 score_mi_device (b200bsp_ctx* c, const float* coeff, float lambda,
     const b200bsp_reg_parms* reg, float* total_score, float* total_grad,
-    float* smetric, int64_t* num_vox)
+    float* smetric, int64_t* num_vox, DevResult* res_host = nullptr,
+    bool waits = false)
 {
     if (c->opts.mi_window == B200BSP_MI_PVI8 && mi_whole_image_pass1 (c) < 0) {
         return fail (c, B200BSP_E_UNSUPPORTED,
@@ -1765,7 +1829,7 @@ score_mi_device (b200bsp_ctx* c, const float* coeff, float lambda,
             "cover the fixed image");
     }
     const float* dcoeff = nullptr;
-    int rc = begin_eval (c, coeff, &dcoeff);
+    int rc = begin_eval (c, coeff, &dcoeff, waits);
     if (rc) return rc;
     rc = mi_passes (c, dcoeff, total_grad, nullptr,
         MI_PASS_HIST | MI_PASS_GRAD);
@@ -1784,10 +1848,10 @@ score_mi_device (b200bsp_ctx* c, const float* coeff, float lambda,
     mi_combine_kernel<<<blocks, 256, 0, c->stream>>> (c->d_res, lambda,
         reg ? c->d_reg_grad64 : nullptr, reg ? c->reg.d_score : nullptr,
         total_grad, n, total_score ? total_score : c->d_total, smetric,
-        (long long*) num_vox);
+        (long long*) num_vox, c->d_err, res_host);
     CK (cudaGetLastError ());
     c->last_launches++;
-    return end_eval (c, false);
+    return waits ? B200BSP_OK : end_eval (c, false);
 }
 
 extern "C" int
@@ -1806,6 +1870,22 @@ b200bsp_score (b200bsp_ctx* c, const float* coeff, int metric_type,
                 total_grad, smetric, num_vox)
             : score_mi_device (c, coeff, lambda, reg, total_score,
                 total_grad, smetric, num_vox);
+    }
+    if ((metric_type == 0 || metric_type == 1) && c->lm_n == 0 && c->h_res_dev) {
+        // the same work with host outputs: scalars through page-locked
+        // memory, the gradient through the staging buffer, one wait
+        float* g_dev = is_device_ptr (total_grad) ? total_grad : c->d_grad;
+        int rc = (metric_type == 0 ? score_mse_device : score_mi_device)
+            (c, coeff, lambda, reg, c->h_scalar, g_dev, nullptr, nullptr,
+            c->h_res_dev, true);
+        if (rc) return rc;
+        if (g_dev == c->d_grad) CK (stage_down (c, total_grad));
+        rc = end_eval (c, true);
+        if (rc) return rc;
+        if (total_score) *total_score = *c->h_scalar;
+        if (smetric) *smetric = c->h_res->score_f;
+        if (num_vox) *num_vox = c->h_res->num_vox;
+        return check_device_error (c, c->h_res->error);
     }
     std::vector<float> g ((size_t) c->num_coeff);
     float s = 0.f;

@@ -141,3 +141,37 @@ def test_line_kernel_field_and_warp(case):
         want = synth.warp_trilinear(moving, fixed, grid, coeff, -7.0).img
         bad = np.abs(w - want) > 0.1
         assert bad.mean() < 1e-4, bad.mean()
+
+
+# below one part of the staged copies (65536 floats), three parts, four
+# longer ones
+@pytest.mark.parametrize("metric", ["mse", "mi"])
+@pytest.mark.parametrize("dim", [(20, 18, 16), (90, 81, 78), (129, 129, 126)])
+def test_score_with_host_outputs_is_the_device_one(dim, metric):
+    """Host coefficients and outputs go through page-locked staging buffers
+    around the same kernels: every bit of the results is the same, also when
+    the host arrays are page-locked themselves."""
+    import ctypes as C
+
+    import torch
+    fixed, moving, grid, coeff = _case(dim, (3, 3, 3), None, 0.0)
+    reg = P.reg_parms(curvature=0.1, total_displacement=0.01)
+    with P.Context(fixed, moving, grid, mi_window="pvi8") as ctx:
+        ctx.set_images()
+        host = ctx.score(coeff, metric, 0.5, reg)
+        pinned = ctx.score(torch.from_numpy(coeff).pin_memory(), metric, 0.5,
+                           reg)
+        dc = torch.from_numpy(coeff).cuda()
+        g = torch.empty_like(dc)
+        s = torch.empty(2, device="cuda")
+        n = torch.empty(1, dtype=torch.int64, device="cuda")
+        rc = P.lib().b200bsp_score(
+            ctx._h, dc.data_ptr(), 0 if metric == "mse" else 1, C.c_float(0.5),
+            C.byref(reg), s.data_ptr(), g.data_ptr(), s.data_ptr() + 4,
+            n.data_ptr())
+        assert rc == 0
+        torch.cuda.synchronize()
+    for got in (host, pinned):
+        assert got[0] == s[0].item() and got[2] == s[1].item()
+        assert got[3] == n.item() and got[3] > 0
+        assert np.array_equal(got[1], g.cpu().numpy())
