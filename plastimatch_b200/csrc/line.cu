@@ -556,6 +556,8 @@ line_kernel (const __grid_constant__ LineArgs a)
     // each thread's own sums
     __shared__ double t_v[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
     __shared__ int t_n[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
+    // (the contraction's blocks may start as this grid's last ones end)
+    if (ln_adjoint (MODE)) asm volatile ("griddepcontrol.launch_dependents;");
     if (ln_mse (MODE)) {
         t_v[threadIdx.x] = 0.0;
         t_n[threadIdx.x] = 0;
@@ -825,11 +827,21 @@ line_kernel (const __grid_constant__ LineArgs a)
 // One block per knot row ky, kxc knots along x and kzc knots along z; a
 // thread owns two voxel columns x, x + 1 of the block's tiles and marches
 // along z (every blockDim.y-th plane), so that every load of a warp is one
-// run of a row.  It contracts along z into a register window of four knots; the knots
-// that leave it meet in shared memory, where they are contracted along x,
-// normalised (MSE) and stored, the block's knots as one run per z knot.  The
-// rows come from L2: what bounds it is how many loads are in flight.  Each block sums the voxel counts for its normalisation; the first
-// one writes the result block.
+// run of a row.  It contracts along z into a register window of four knots;
+// the knots that leave it meet in shared memory, where they are contracted
+// along x, normalised (MSE) and stored, the block's knots as one run per z
+// knot.  The rows come from L2: what bounds it is how many loads are in
+// flight.  (The next planes' loads sent out before the last ones are used:
+// 88 us a call at 256x256x128 vpr 5 where this takes 83; the registers for
+// it leave fewer planes in flight.)  Each block sums the voxel counts for
+// its normalisation; the first one writes the result block.
+//
+// Its launch does not wait for the end of the line kernel's: the blocks
+// start as the last of that one's end, fetch the weights and wait there
+// (64^3 vpr 8: 14.6 us a call where one after the other takes 18.3).  The
+// rows, counts and scores are written during this kernel's lifetime then:
+// they are read through L2, never as read-only data.
+
 constexpr int LF_MAX_THREADS = 512;
 
 struct LineFinishArgs {
@@ -852,8 +864,10 @@ struct LineFinishArgs {
 };
 
 // NZ2: planes of a tile in flight where at most two y blocks reach a row.
-template <int NZ2>
-__global__ void __launch_bounds__ (LF_MAX_THREADS)
+// MIN_BLOCKS: blocks an SM holds (2: of at most 320 threads).
+template <int NZ2, int MIN_BLOCKS>
+__global__ void
+__launch_bounds__ (MIN_BLOCKS == 1 ? LF_MAX_THREADS : 320, MIN_BLOCKS)
 line_finish_kernel (const __grid_constant__ LineFinishArgs a)
 {
     extern __shared__ __align__ (16) float sh[];       // [part][c][kz][voxel]
@@ -861,7 +875,6 @@ line_finish_kernel (const __grid_constant__ LineFinishArgs a)
     __shared__ ulonglong2 sbz[2 * 64];                 // each weight twice
     __shared__ double sh_v[LF_MAX_THREADS / 32];
     __shared__ int sh_n[LF_MAX_THREADS / 32];
-    __shared__ long long s_n;
     const BspGeom& g = a.g;
     const int vx = g.vpr[0], vy = g.vpr[1], vz = g.vpr[2];
     const int T = blockDim.x, P = blockDim.y, NT = T * P;
@@ -876,6 +889,7 @@ line_finish_kernel (const __grid_constant__ LineFinishArgs a)
         ((u64*) sbz)[o] = pk (w, w);
     }
     __syncthreads ();
+    asm volatile ("griddepcontrol.wait;" ::: "memory");
 
     // tile rows along z that reach the block's knots, y blocks that reach ky
     const int ta = max (0, kz0 - 3), tb = min (g.rdims[2], kz0 + nkz);
@@ -930,7 +944,7 @@ line_finish_kernel (const __grid_constant__ LineFinishArgs a)
                         const float* rb = r + b * ys;
 #pragma unroll
                         for (int c = 0; c < 3; c++, rb += a.nxs) {
-                            e[q][b][c] = in ? __ldg ((const u64*) rb) : 0ull;
+                            e[q][b][c] = in ? __ldcg ((const u64*) rb) : 0ull;
                         }
                     }
                     r += pstep;
@@ -963,71 +977,73 @@ line_finish_kernel (const __grid_constant__ LineFinishArgs a)
     leave (tb);
     leave (tb + 1);
     leave (tb + 2);
-
-    // the voxel count (and on the first block the score), in index order
+    // The blocks' counts (and on the first block their scores), in index order
     const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-    double v = 0.0;
-    int n32 = 0;
-    for (int i0 = tid; i0 < a.nparts; i0 += 4 * NT) {
-        int c4[4];
-        double s4[4];
+    {
+        double v = 0.0;
+        int n32 = 0;
+        for (int i0 = tid; i0 < a.nparts; i0 += 4 * NT) {
+            int c4[4];
+            double s4[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int i = i0 + u * NT;
-            c4[u] = i < a.nparts ? __ldg (a.cp + i) : 0;
-            s4[u] = first && i < a.nparts ? __ldg (a.sp + i) : 0.0;
+            for (int u = 0; u < 4; u++) {
+                const int i = i0 + u * NT;
+                c4[u] = i < a.nparts ? __ldcg (a.cp + i) : 0;
+                s4[u] = first && i < a.nparts ? __ldcg (a.sp + i) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                n32 += c4[u];
+                v += s4[u];
+            }
         }
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            n32 += c4[u];
-            v += s4[u];
+        for (int o = 16; o > 0; o >>= 1) {
+            v += __shfl_down_sync (0xffffffffu, v, o);
+            n32 += __shfl_down_sync (0xffffffffu, n32, o);
         }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v += __shfl_down_sync (0xffffffffu, v, o);
-        n32 += __shfl_down_sync (0xffffffffu, n32, o);
-    }
-    if ((tid & 31) == 0) {
-        sh_v[tid >> 5] = v;
-        sh_n[tid >> 5] = n32;
+        if ((tid & 31) == 0) {
+            sh_v[tid >> 5] = v;
+            sh_n[tid >> 5] = n32;
+        }
     }
     __syncthreads ();
-    if (tid == 0) {
-        for (int w = 1; w < NT / 32; w++) {
-            v += sh_v[w];
-            n32 += sh_n[w];
-        }
+
+    long long n_all = 0;
+    if (a.nparts > 0) {
+        int n32 = 0;
+        for (int w = 0; w < NT / 32; w++) n32 += sh_n[w];
+        n_all = n32;
+    }
+    if (first && tid == 0) {
         DevResult r;
         if (a.nparts > 0) {
+            double v = 0.0;
+            for (int w = 0; w < NT / 32; w++) v += sh_v[w];
             r.raw = v;
-            r.num_vox = n32;
+            r.num_vox = n_all;
             r.error = a.err ? *a.err : 0;
-            r.score = n32 < 1 ? (double) FLT_MAX : v / (double) n32;
-            r.score_f = n32 < 1 ? FLT_MAX : (float) r.score;
+            r.score = n_all < 1 ? (double) FLT_MAX : v / (double) n_all;
+            r.score_f = n_all < 1 ? FLT_MAX : (float) r.score;
+            *a.res = r;
         } else {
             r = *a.res;
         }
-        s_n = r.num_vox;
-        if (first) {
-            if (a.nparts > 0) *a.res = r;
-            if (a.res_host) *a.res_host = r;
-            if (a.cb.total_score) {
-                // Bspline_score::accumulate then the regulariser's score
-                // (src/register/bspline.cxx:595-622), in float
-                float total = 0.f;
-                total += a.cb.lambda * r.score_f;
-                if (a.cb.reg_score) total += (float) *a.cb.reg_score;
-                *a.cb.total_score = total;
-            }
-            if (a.score_out) *a.score_out = r.score_f;
-            if (a.score64_out) *a.score64_out = r.score;
-            if (a.nvox_out) *a.nvox_out = r.num_vox;
+        if (a.res_host) *a.res_host = r;
+        if (a.cb.total_score) {
+            // Bspline_score::accumulate then the regulariser's score
+            // (src/register/bspline.cxx:595-622), in float
+            float total = 0.f;
+            total += a.cb.lambda * r.score_f;
+            if (a.cb.reg_score) total += (float) *a.cb.reg_score;
+            *a.cb.total_score = total;
         }
+        if (a.score_out) *a.score_out = r.score_f;
+        if (a.score64_out) *a.score64_out = r.score;
+        if (a.nvox_out) *a.nvox_out = r.num_vox;
     }
-    __syncthreads ();
     const double scale = a.nparts == 0 ? 1.0
-        : s_n < 1 ? 0.0 : 2.0 / (double) s_n;
+        : n_all < 1 ? 0.0 : 2.0 / (double) n_all;
     // the parts' sums, into the first
     if (P > 1) {
         for (int o = tid; o < 3 * hs; o += NT) {
@@ -1296,7 +1312,7 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     const float* luts, const double* score_part, const int* count_part,
     int nparts, const int* err, DevResult* res, DevResult* res_host,
     float* grad, double* grad64, float* score_out, double* score64_out,
-    long long* nvox_out, cudaStream_t st, const FinishCombine& cb)
+    long long* nvox_out, cudaStream_t st, const FinishCombine& cb, bool behind)
 {
     LineFinishArgs a;
     a.g = g;
@@ -1323,34 +1339,61 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     const int nbx = (g.cdims[0] + most - 1) / most;
     a.kxc = (g.cdims[0] + nbx - 1) / nbx;
     const int threads = (((a.kxc + 3) * g.vpr[0] + 2) / 2 + 31) / 32 * 32;
-    // knots along z: a block reads 3 tile rows beyond its own, so few large
-    // blocks read less, but it takes some 300 to fill the chip (512x512x160:
-    // 36 us with 8, 44 with 4; 256x256x128: 13 with 4, 17 with 8); grids
-    // with fewer knots split a tile's planes over more threads
-    a.kzc = 8;
-    auto blocks = [&] () {
-        return nbx * g.cdims[1] * ((g.cdims[2] + a.kzc - 1) / a.kzc);
-    };
-    while (a.kzc > 2 && blocks () < 300) a.kzc /= 2;
-    int parts = 1;
-    while (parts < 4 && parts < g.vpr[2] && threads * (parts + 1) <= 256
-           && blocks () * threads * parts < 148 * 512) {
-        parts++;
+    // Knots along z a block, and parts its tiles' planes are split over: of
+    // the splits whose blocks are all resident at once (512 threads of 128
+    // registers an SM) the one with the shortest march, a block's own tile
+    // rows and the 3 beyond them times a latency and its planes.  Against 2
+    // to 8 knots and 1 to 4 parts by the number of blocks alone (some 300),
+    // the call takes at 131x117x83 vpr 6 25.7 us where that took 27.1, at
+    // 200x180x90 vpr 7x7x4 with ROIs 48.3 (51.5: 377 blocks of which 296
+    // were resident), eight uneven images 308 (317).  Where no split is
+    // resident (512x512x160) the row of 8 knots reads least: 343 us, 347
+    // with 5, 356 with 2; two blocks an SM in 96 registers, one in 128: 352.
+    double best = 0.0;
+    int parts = 0;
+    for (int kzc = 1; kzc <= 8; kzc++) {
+        const int n = nbx * g.cdims[1] * ((g.cdims[2] + kzc - 1) / kzc);
+        for (int p = 1; p <= std::min (g.vpr[2], 8); p++) {
+            if (p * threads > LF_MAX_THREADS
+                || n > 148 * (LF_MAX_THREADS / (p * threads))) break;
+            const double cost = (kzc + 3)
+                * (0.6 + 0.2 * ((g.vpr[2] + p - 1) / p));
+            if (parts && cost >= best) continue;
+            best = cost;
+            parts = p;
+            a.kzc = kzc;
+        }
+    }
+    const bool waves = parts == 0;
+    if (waves) {
+        a.kzc = 8;
+        parts = 1;
     }
     const dim3 grid (nbx, g.cdims[1], (g.cdims[2] + a.kzc - 1) / a.kzc);
     const size_t smem = (size_t) 6 * a.kzc * threads * parts * sizeof (float);
     // the fewest rounds of at most five planes, evenly filled
     const int nz = (g.vpr[2] + parts - 1) / parts;
     const int rounds = (nz + 4) / 5;
-    auto k = line_finish_kernel<5>;
-    if ((nz + rounds - 1) / rounds <= 3) k = line_finish_kernel<3>;
-    else if ((nz + rounds - 1) / rounds == 4) k = line_finish_kernel<4>;
+    const int most_nz = (nz + rounds - 1) / rounds;
+    auto k = line_finish_kernel<5, 1>;
+    if (waves && threads <= 320 && most_nz <= 4) k = line_finish_kernel<4, 2>;
+    else if (most_nz <= 3) k = line_finish_kernel<3, 1>;
+    else if (most_nz == 4) k = line_finish_kernel<4, 1>;
     if (smem > LN_PLAIN_SMEM) {
         cudaError_t e = set_max_dynamic_smem ((const void*) k, (int) smem);
         if (e != cudaSuccess) return e;
     }
-    k<<<grid, dim3 (threads, parts), smem, st>>> (a);
-    return cudaGetLastError ();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3 (threads, parts);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = behind ? 1 : 0;
+    return cudaLaunchKernelEx (&cfg, k, a);
 }
 
 } // namespace b200

@@ -61,12 +61,14 @@ cudaError_t launch_field_line (const BspGeom& g, const LinePlan& p,
 
 // Contraction of the adjoint rows into the gradient, score and count over
 // the nparts block parts (0: the result block stands, no normalisation), as
-// launch_finish_mse otherwise.
+// launch_finish_mse otherwise.  behind: the kernel that writes the rows is
+// the last work on the stream and nothing else has to be waited for, so that
+// this one may be launched before that one has ended.
 cudaError_t launch_line_finish (const BspGeom& g, const LinePlan& p,
     const float* rows, const float* luts, const double* score_part,
     const int* count_part, int nparts, const int* err, DevResult* res,
     DevResult* res_host, float* grad, double* grad64, float* score_out,
     double* score64_out, long long* nvox_out, cudaStream_t st,
-    const FinishCombine& cb = FinishCombine ());
+    const FinishCombine& cb, bool behind);
 
 } // namespace b200

@@ -1025,7 +1025,7 @@ mi_run_line (MiState* s, const BspGeom& g, const LinePlan& plan,
             != cudaSuccess
         || launch_line_finish (g, plan, rows, d_luts, nullptr, nullptr, 0,
             nullptr, d_res, nullptr, grad_out, grad64_out, nullptr, nullptr,
-            nullptr, st) != cudaSuccess) {
+            nullptr, st, FinishCombine (), true) != cudaSuccess) {
         return B200BSP_E_CUDA;
     }
     if (launches) *launches += 3;

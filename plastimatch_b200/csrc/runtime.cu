@@ -1033,7 +1033,7 @@ run_mse (b200bsp_ctx* c, const float* dcoeff, float* grad_out,
         CK (launch_line_finish (g, c->lplan, c->d_rows, c->d_luts,
             c->d_score_part, c->d_count_part, c->lplan.nblocks, c->d_err,
             c->d_res, res_host, grad_out, grad64_out, score_out, score64_out,
-            nvox_out, c->stream, combine));
+            nvox_out, c->stream, combine, !before_finish));
         c->last_launches += 1;
         return B200BSP_OK;
     }

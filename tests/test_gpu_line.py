@@ -37,6 +37,11 @@ CASES = [
 # arrays beside it need the larger limit
 LARGE_BLOCKS = [((224, 529, 28), (3, 3, 9), None, 0.0),
                 ((81, 439, 106), (4, 3, 10), None, 0.0)]
+# more blocks of the rows' contraction than the chip holds at once, of two
+# and of one block an SM; one part a tile and eight
+CONTRACTIONS = [((300, 590, 40), (10, 3, 4), None, 0.0),
+                ((300, 590, 50), (10, 3, 5), None, 0.0),
+                ((40, 44, 81), (4, 10, 9), None, 0.0)]
 
 
 def _volume(dim, seed, dcos, origin=(0.0, 0.0, 0.0)):
@@ -58,7 +63,7 @@ def _case(dim, vpr, roi, angle, seed=71):
 
 
 @pytest.mark.parametrize("grad", ["nearest", "trilinear"])
-@pytest.mark.parametrize("case", CASES + LARGE_BLOCKS)
+@pytest.mark.parametrize("case", CASES + LARGE_BLOCKS + CONTRACTIONS)
 def test_line_kernel_matches_tile_kernel(case, grad):
     fixed, moving, grid, coeff = _case(*case)
     out = []
