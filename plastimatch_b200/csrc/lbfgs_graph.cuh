@@ -11,8 +11,8 @@ namespace b200 {
 // Start of a line search (after the correction pair, the two-loop
 // recursion and gp.d): the search's state and its first trial step; ends
 // the run (h_while) when the step or the direction is unusable.  dginit is
-// the sum of slot LP_DG0 of part (nparts partials per slot), or, with part
-// NULL, already in s.  Launched with one warp.
+// the sum of slot LP_DG0 of part (nparts partials per slot).  Launched with
+// one warp.
 __global__ void lb_begin_search_kernel (LbDev* s,
     cudaGraphConditionalHandle h_while, const double* part, int nparts);
 
@@ -23,5 +23,15 @@ __global__ void lb_begin_search_kernel (LbDev* s,
 __global__ void lb_after_eval_kernel (LbDev* s,
     cudaGraphConditionalHandle h_while, cudaGraphConditionalHandle h_new,
     const double* part, int nparts);
+
+// The new-line-search branch, and the work after an evaluation, as one
+// launch each; for vectors of at most LB_CLUSTER_MAX entries.
+constexpr long long LB_CLUSTER_MAX = 1 << 16;
+cudaError_t launch_lb_search (LbDev* dst, cudaGraphConditionalHandle h_while,
+    double* S, double* Y, const double* x, double* xp, const double* g,
+    double* gp, double* d, double* dsc, long long n, cudaStream_t st);
+cudaError_t launch_lb_eval (LbDev* dst, cudaGraphConditionalHandle h_while,
+    cudaGraphConditionalHandle h_new, const float* grad, double* g,
+    const double* d, const double* x, long long n, cudaStream_t st);
 
 }  // namespace b200

@@ -596,101 +596,6 @@ lb_j2 (const LbDev* s, int i)
     return (s->end - s->bound + i + 2 * s->m) % s->m;
 }
 
-// The whole new-line-search branch in one block, for vectors of at most
-// LB_FUSED_MAX entries: correction pair, the two-loop recursion, xp = x,
-// gp = g and dginit = gp.d, each dot product a block reduction in a fixed
-// order (one launch instead of some fifty for small registrations).
-constexpr long long LB_FUSED_MAX = 1 << 17;
-constexpr int LB_FUSED_THREADS = 1024;
-
-__device__ double
-lb_block_dot (const double* __restrict__ a, const double* __restrict__ b,
-    long long n, double* red)
-{
-    double s = 0.0;
-    for (long long i = threadIdx.x; i < n; i += LB_FUSED_THREADS) s += a[i] * b[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync (0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads ();
-    if (threadIdx.x < 32) {
-        double v = red[threadIdx.x];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync (0xffffffffu, v, o);
-        if (threadIdx.x == 0) red[32] = v;
-    }
-    __syncthreads ();
-    const double r = red[32];
-    __syncthreads ();
-    return r;
-}
-
-__global__ void __launch_bounds__ (LB_FUSED_THREADS)
-lb_branch_fused_kernel (const LbDev* __restrict__ st, double* __restrict__ S,
-    double* __restrict__ Y, const double* __restrict__ x,
-    double* __restrict__ xp, const double* __restrict__ g,
-    double* __restrict__ gp, double* __restrict__ d,
-    double* __restrict__ dsc, double* __restrict__ dginit, long long n)
-{
-    __shared__ double red[33];
-    const int m = st->m;
-    const bool first = st->first;
-    const int t = threadIdx.x;
-    if (!first) {
-        double* sn = S + (size_t) st->newest * n;
-        double* yn = Y + (size_t) st->newest * n;
-        for (long long i = t; i < n; i += LB_FUSED_THREADS) {
-            sn[i] = x[i] - xp[i];
-            yn[i] = g[i] - gp[i];
-        }
-        __syncthreads ();
-        const double ys = lb_block_dot (yn, sn, n, red);
-        const double yy = lb_block_dot (yn, yn, n, red);
-        if (t == 0) {
-            dsc[st->newest] = ys;
-            dsc[2 * m + 1] = yy;
-        }
-    }
-    for (long long i = t; i < n; i += LB_FUSED_THREADS) d[i] = -1.0 * g[i] + 0.0 * d[i];
-    __syncthreads ();
-    if (!first) {
-        const int bound = st->bound;
-        int j = st->end;
-        for (int k = 0; k < bound; k++) {
-            j = (j + m - 1) % m;
-            const double* sj = S + (size_t) j * n;
-            const double* yj = Y + (size_t) j * n;
-            const double alpha = lb_block_dot (sj, d, n, red) / dsc[j];
-            if (t == 0) dsc[m + j] = alpha;
-            for (long long i = t; i < n; i += LB_FUSED_THREADS) {
-                d[i] = (-1.0 * alpha) * yj[i] + 1.0 * d[i];
-            }
-            __syncthreads ();
-        }
-        const double bv = dsc[st->newest] / dsc[2 * m + 1];
-        for (long long i = t; i < n; i += LB_FUSED_THREADS) d[i] = 0.0 * d[i] + bv * d[i];
-        __syncthreads ();
-        for (int k = 0; k < bound; k++) {
-            const double* sj = S + (size_t) j * n;
-            const double* yj = Y + (size_t) j * n;
-            const double beta = lb_block_dot (yj, d, n, red) / dsc[j];
-            const double av = dsc[m + j] - beta;
-            for (long long i = t; i < n; i += LB_FUSED_THREADS) {
-                d[i] = av * sj[i] + 1.0 * d[i];
-            }
-            __syncthreads ();
-            j = (j + 1) % m;
-        }
-    }
-    for (long long i = t; i < n; i += LB_FUSED_THREADS) {
-        xp[i] = x[i];
-        gp[i] = g[i];
-    }
-    __syncthreads ();
-    const double dg0 = lb_block_dot (gp, d, n, red);
-    if (t == 0) *dginit = dg0;
-}
-
 // x = xp + stp d (the trial point) and its float copy, the evaluation's
 // coefficients; both stay when the run is over (the float copy already
 // holds x then)
@@ -971,13 +876,17 @@ build_lbfgs_graph (b200bsp_ctx* ctx, Lbfgs& w, LbDev* dst, int metric,
     }
     const int m = w.m;
     double* ys_d = w.dsc;
-    // the new-line-search branch
-    if (ok && n <= LB_FUSED_MAX && cudaStreamBeginCaptureToGraph (st, branch,
+    // the new-line-search branch: one cluster for vectors that its threads'
+    // registers hold (ten iterations, 13 evaluations at 64^3: vpr 8, 3993
+    // entries, 965 us; vpr 3, 46875 entries, 1265), the chain below beyond
+    // (81^3 vpr 3, 81000 entries: 1983 us).  One block for all of it, its
+    // vectors from L2 at every step, took 1187, 3270 and 4790.
+    if (ok && n <= LB_CLUSTER_MAX && cudaStreamBeginCaptureToGraph (st, branch,
             nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
-        lb_branch_fused_kernel<<<1, LB_FUSED_THREADS, 0, st>>> (dst, w.s, w.y,
-            w.x, w.xp, w.g, w.gp, w.d, ys_d, &dst->dginit, n);
-        lb_begin_search_kernel<<<1, 32, 0, st>>> (dst, h_while, nullptr, 0);
-        ok = cudaStreamEndCapture (st, &out) == cudaSuccess && out == branch;
+        const bool launched = launch_lb_search (dst, h_while, w.s, w.y, w.x,
+            w.xp, w.g, w.gp, w.d, ys_d, n, st) == cudaSuccess;
+        ok = cudaStreamEndCapture (st, &out) == cudaSuccess && out == branch
+            && launched;
     } else if (ok && cudaStreamBeginCaptureToGraph (st, branch, nullptr,
             nullptr, 0, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
         // the correction pair, the two-loop recursion, xp, gp and gp.d:
@@ -1009,12 +918,18 @@ build_lbfgs_graph (b200bsp_ctx* ctx, Lbfgs& w, LbDev* dst, int metric,
         // regulariser)
         const int rc = b200bsp_score (ctx, coeff_f, metric, lambda, reg,
             &dst->total, grad_f, nullptr, nullptr);
-        lb_eval_dots_kernel<<<OPT_BLOCKS, OPT_THREADS, 0, st>>> (grad_f, w.g,
-            w.d, w.x, n, w.part);
-        lb_after_eval_kernel<<<1, 32, 0, st>>> (dst, h_while, h_new, w.part,
-            OPT_BLOCKS);
+        bool launched = true;
+        if (n <= LB_CLUSTER_MAX) {
+            launched = launch_lb_eval (dst, h_while, h_new, grad_f, w.g, w.d,
+                w.x, n, st) == cudaSuccess;
+        } else {
+            lb_eval_dots_kernel<<<OPT_BLOCKS, OPT_THREADS, 0, st>>> (grad_f,
+                w.g, w.d, w.x, n, w.part);
+            lb_after_eval_kernel<<<1, 32, 0, st>>> (dst, h_while, h_new,
+                w.part, OPT_BLOCKS);
+        }
         ok = cudaStreamEndCapture (st, &out) == cudaSuccess && out == body
-            && rc == B200BSP_OK;
+            && rc == B200BSP_OK && launched;
     } else {
         ok = false;
     }

@@ -144,3 +144,19 @@ def _compare_graph_and_host(case, form, vpr, with_reg, metric="mse"):
     assert r_g["status"] == r_h["status"], (r_g, r_h)
     assert abs(r_g["score"] - r_h["score"]) <= 1e-5 * abs(r_h["score"])
     assert np.linalg.norm(c_g - c_h) <= 1e-4 * max(np.linalg.norm(c_h), 1.0)
+
+
+# entries of the vectors: one block's, several blocks of a cluster, more
+# entries a thread, beyond what a cluster takes
+@pytest.mark.parametrize("dim,vpr", [(64, 8), (40, 4), (64, 5), (64, 3), (81, 3)])
+def test_graph_step_sizes_match_host_loop(dim, vpr):
+    """The line search's start and the work after an evaluation take one
+    cluster, sized by the number of coefficients, or launches of their own
+    beyond it: the same run as the host-driven loop's, whose dot products
+    differ in the order of their double sums only (bars as above)."""
+    fixed = synth.gaussian_blobs((dim, dim, dim), spacing=(1.0, 1.1, 1.3),
+                                 seed=20261211)
+    g0 = BsplineGrid.for_volume(fixed, 8)
+    moving = synth.warp_trilinear(fixed, fixed, g0,
+                                  synth.random_coeff(g0, 2.0, 20261212))
+    _compare_graph_and_host((fixed, moving), "tc", vpr, False)
