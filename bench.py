@@ -76,9 +76,16 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
+# by the kernel that ran the timed evaluations
+TC_SPLITS = ("voxel work f32; tensor-core products as 3-term bf16 splits with "
+             "f32 accumulation")
+ARITHMETIC = {"line": "f32 (packed pairs), score sums f64",
+              "tile": TC_SPLITS, "xlane": TC_SPLITS}
+
+
 def profile_traffic(kernel):
-    """ncu DRAM bytes per launch of the kernel that ran ("tile", "xlane" or
-    "fp32", as b200bsp_mse_kernel names it)."""
+    """ncu DRAM bytes per launch of the kernel that ran ("line", "tile",
+    "xlane" or "fp32", as b200bsp_mse_kernel names it)."""
     p = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(p):
         with open(p) as f:
@@ -406,7 +413,7 @@ def extra_metrics(P, ctx, stream, flush, d_coeff, d_grad, nvox, warmup,
 
     def mse_reg():
         # bspline_score with device outputs: the regulariser overlaps the
-        # tile kernel on the context's second stream
+        # MSE kernel on the context's second stream
         rc = lib.b200bsp_score(ctx._h, d_coeff.data_ptr(), 0, C.c_float(1.0),
                                C.byref(reg), d_total.data_ptr(),
                                d_grad.data_ptr(), d_total[1:].data_ptr(),
@@ -450,7 +457,7 @@ def measure_form(P, form, args, workload, local_rank, dist, flush,
 
     Returns a dict: device ms per evaluation (CUDA events on the context's
     stream, L2 flushed before every step and excluded, max over ranks),
-    end-to-end ms through the C ABI with pinned host buffers, the tile
+    end-to-end ms through the C ABI with pinned host buffers, the MSE
     kernel's own ms (the library's events, median of three probes), the
     launches per evaluation, the autotuned tiles per batch, and the last
     evaluation's score, gradient and voxel count (host copies)."""
@@ -851,10 +858,8 @@ def main():
             "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic",
             "config": dict(WORKLOAD, form=args.form,
-                           arithmetic="voxel work f32; tensor-core products "
-                                      "as 3-term bf16 splits with f32 "
-                                      "accumulation" if args.form == "tc"
-                                      else "f32 SIMT",
+                           arithmetic=ARITHMETIC.get(m["kernel"][0],
+                                                     "f32 SIMT"),
                            l2="inputs 167 MB > L2 and 256 MiB flush write "
                               "before every timed step (excluded)",
                            parallelism=f"replicas x{world}",
