@@ -599,6 +599,23 @@ line_kernel (const __grid_constant__ LineArgs a)
         for (int o = threadIdx.x; o < a.bins * a.bins; o += blockDim.x) slut[o] = a.lut[o];
     }
     const float scale = MODE == LN_PZ_GRAD ? a.nvf[1] : 0.f;
+    // the block's coefficients contracted along z, for each of its planes;
+    // their loads go out before the weights are waited for (256x256x128
+    // vpr 5: 82.3 us a call, 83.3 after them)
+    const int plane = 3 * g.cdims[0] * g.cdims[1];
+    float ck[4][3];
+    auto fetch = [&] (int o) {
+        const int jj = o / nkx, i = o - jj * nkx;
+        const float* c = a.coeff + 3 * ((size_t) (tz * g.cdims[1] + ty0 + jj)
+            * g.cdims[0] + t0 + i);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#pragma unroll
+            for (int d = 0; d < 3; d++) ck[k][d] = __ldg (c + (size_t) k * plane + d);
+        }
+    };
+    int oc = threadIdx.x;
+    if (oc < nj * nkx) fetch (oc);
     for (int o = threadIdx.x; o < 4 * vx; o += blockDim.x) {
         const float w = a.luts[o];
         sbx[o] = pk (w, w);
@@ -607,31 +624,20 @@ line_kernel (const __grid_constant__ LineArgs a)
         sbz[o] = a.luts[4 * (vx + vy) + o];
     }
     __syncthreads ();
-    // the block's coefficients contracted along z, for each of its planes
-    {
-        const int plane = 3 * g.cdims[0] * g.cdims[1];
-        for (int o = threadIdx.x; o < nj * nkx; o += blockDim.x) {
-            const int jj = o / nkx, i = o - jj * nkx;
-            const float* c = a.coeff + 3 * ((size_t) (tz * g.cdims[1] + ty0 + jj)
-                * g.cdims[0] + t0 + i);
-            float ck[4][3];
+    while (oc < nj * nkx) {
+        for (int z = 0; z < nz; z++) {
+            const float4 w = *(const float4*) (sbz + 4 * z);
+            float v[3];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-#pragma unroll
-                for (int d = 0; d < 3; d++) ck[k][d] = __ldg (c + (size_t) k * plane + d);
+            for (int d = 0; d < 3; d++) {
+                v[d] = fmaf (w.w, ck[3][d], fmaf (w.z, ck[2][d],
+                    fmaf (w.y, ck[1][d], w.x * ck[0][d])));
             }
-            for (int z = 0; z < nz; z++) {
-                const float4 w = *(const float4*) (sbz + 4 * z);
-                float v[3];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    v[d] = fmaf (w.w, ck[3][d], fmaf (w.z, ck[2][d],
-                        fmaf (w.y, ck[1][d], w.x * ck[0][d])));
-                }
-                cz[(z * nj + jj) * nkx + i] = make_ulonglong2 (pk (v[0], v[1]),
-                    pk (v[2], 0.f));
-            }
+            cz[z * nj * nkx + oc] = make_ulonglong2 (pk (v[0], v[1]),
+                pk (v[2], 0.f));
         }
+        oc += blockDim.x;
+        if (oc < nj * nkx) fetch (oc);
     }
 
     // the thread's column (a lane beyond the ROI stays on valid addresses)
