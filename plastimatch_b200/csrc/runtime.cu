@@ -1738,10 +1738,12 @@ b200bsp_landmarks_score (b200bsp_ctx* c, const float* coeff, float* lmetric,
 // bspline_score with MSE and device outputs, stream-ordered: the MSE
 // kernel, the regulariser's passes beside it on the context's second
 // stream, then the finish kernel that combines them (lambda times the
-// metric, plus the regulariser's score and double gradient).  The MSE
-// kernel holds every register of the SMs it runs on, so it is launched on
-// all but REG_SIDE_SMS of them and the passes (a few microseconds of work
-// each, but three dependent launches) run on the rest meanwhile.
+// metric, plus the regulariser's score and double gradient).  A persistent
+// MSE kernel holds every register of the SMs it runs on, so it is launched
+// on all but REG_SIDE_SMS of them and the passes (a few microseconds of work
+// each, but three dependent launches) run on the rest meanwhile.  The line
+// kernel's blocks leave room as they end: 256x256x128 vpr 5 120.7 us, in
+// stream order 126.4; 64^3 vpr 8 37.2 and 41.1.
 static int
 score_mse_device (b200bsp_ctx* c, const float* coeff, float lambda,
     const b200bsp_reg_parms* reg, float* total_score, float* total_grad,
