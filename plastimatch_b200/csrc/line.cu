@@ -37,6 +37,7 @@
 
 #include "bsp_common.cuh"
 #include "line.cuh"
+#include "line_index.cuh"
 
 namespace b200 {
 
@@ -108,7 +109,7 @@ struct LineArgs {
     u64 step_y;          // AXIS: (0, fixed y step)
     u64 morg, mprj;      // AXIS: moving x and y origin and projection
     int mtop[3];         // bits of 2^23 + (dim - 2): the largest corner
-    int midx0;           // index of corner bits (0, 0, 0) (mod 2^32)
+    unsigned midx0;      // line_corner0 of the moving image
 };
 
 __device__ __forceinline__ u64
@@ -281,8 +282,7 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
             v.clamp |= 1 << d;
         }
     }
-    const int mvf = bits[0] + g.mdim[0] * (bits[1] + g.mdim[1] * bits[2])
-        + a.midx0;
+    const unsigned mvf = line_corner (bits, g.mdim[0], g.mdim[1], a.midx0);
     const int fidx = col.frow + fj * g.fdim[0];
     v.fidx = fidx;
     if (MODE == LN_FIELD) {
@@ -297,23 +297,23 @@ line_load (const LineArgs& a, const Col<AXIS>& col, int fj, u64& jf2,
         // mask lies on the moving image's own grid its index is the clamped
         // floor of the position (the same operations as inside_roi)
         if (AXIS && a.roi_same) {
-            v.roi = __ldg (g.mroi + (rbits[0] + g.mdim[0] * (rbits[1]
-                + g.mdim[1] * rbits[2]) + a.midx0));
+            v.roi = __ldg (g.mroi + line_corner (rbits, g.mdim[0], g.mdim[1],
+                a.midx0));
         } else {
             const float dd[3] = {lo2 (dxy), hi2 (dxy), dz};
             v.roi = roi_moving_ok (g, fx, dd);
         }
     }
     const int dx = g.mdim[0], dxym = g.mdim[0] * g.mdim[1];
-    const unsigned off = (unsigned) mvf * 4u;
+    const unsigned off = mvf * 4u;
     const char* b0 = (const char*) a.mimg;
     const char* b1 = (const char*) (a.mimg + dx);
     const char* b2 = (const char*) (a.mimg + dxym);
     const char* b3 = (const char*) (a.mimg + dxym + dx);
     if (MODE == LN_MSE_NEAREST) {
-        const int mvr = mvf + (v.w2[0] >= 0.5f ? 1 : 0)
+        const unsigned mvr = mvf + (v.w2[0] >= 0.5f ? 1 : 0)
             + (v.w2[1] >= 0.5f ? dx : 0) + (v.w2[2] >= 0.5f ? dxym : 0);
-        const float* gp = a.mgrad + 3 * (size_t) (unsigned) mvr;
+        const float* gp = a.mgrad + 3 * (size_t) mvr;
         v.gr[0] = ld1 (gp);
         v.gr[1] = ld1 (gp + 1);
         v.gr[2] = ld1 (gp + 2);
@@ -1196,9 +1196,8 @@ line_args (const BspGeom& g, const LinePlan& p, const float* coeff,
     a.step_y = two (0.f, g.fstep[4]);
     a.morg = two (g.morigin[0], g.morigin[1]);
     a.mprj = two (g.mproj[0], g.mproj[4]);
-    for (int d = 0; d < 3; d++) a.mtop[d] = 0x4B000000 + g.mdim[d] - 2;
-    a.midx0 = (int) (0u - 0x4B000000u * (1u + (unsigned) g.mdim[0]
-        * (1u + (unsigned) g.mdim[1])));
+    for (int d = 0; d < 3; d++) a.mtop[d] = (int) LINE_BIAS + g.mdim[d] - 2;
+    a.midx0 = line_corner0 (g.mdim[0], g.mdim[1]);
 }
 
 template <int MODE, bool AXIS, bool ROI>
