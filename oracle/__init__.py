@@ -106,6 +106,11 @@ def port():
     return _port
 
 
+class ReferenceNotBuilt(RuntimeError):
+    """A call into the reference library, which is built from the reference's
+    source tree and absent where there is none."""
+
+
 def ref_available() -> bool:
     return os.path.exists(REF_SO)
 
@@ -114,8 +119,8 @@ def ref():
     global _ref
     if _ref is None:
         if not ref_available():
-            raise RuntimeError("oracle/_ref/libplmref.so not built "
-                               "(oracle/build_ref.sh)")
+            raise ReferenceNotBuilt("oracle/_ref/libplmref.so not built "
+                                    "(oracle/build_ref.sh)")
         _ref = C.CDLL(REF_SO)
     return _ref
 

@@ -16,6 +16,17 @@ def pytest_configure(config):
         "markers", "gpu: needs a CUDA device (B200, sm_100a)")
 
 
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_call(item):
+    """A test that calls the reference library is skipped where the library
+    cannot be built (no reference source tree)."""
+    outcome = yield
+    from oracle import ReferenceNotBuilt
+    if outcome.excinfo and issubclass(outcome.excinfo[0], ReferenceNotBuilt):
+        outcome.force_exception(
+            pytest.skip.Exception(str(outcome.excinfo[1])))
+
+
 def golden_names(prefix=""):
     return sorted(f[:-4] for f in os.listdir(GOLDEN)
                   if f.endswith(".npz") and f.startswith(prefix))
