@@ -88,11 +88,12 @@ typedef struct {
  * separable, marching along y) on grids with 3 to 10 voxels a region on
  * every axis, with or without image ROIs, for every evaluation but the
  * optimiser's (which amplifies the last bits of a gradient and keeps to the
- * tensor-core kernels).  There, and on other grids, it starts on the
- * tile kernel (the voxels of one tile on the TMEM lanes); b200bsp_autotune
- * may move it to the x-lane kernel (voxel x on the lanes, 3 <=
- * vox_per_rgn[1] <= 10) and back, and image ROIs (b200bsp_set_roi) move it
- * to the x-lane kernel.  XLANE and TILE pin one of the tensor-core kernels
+ * tensor-core kernels).  There, on other grids, and on a device that lacks
+ * the memory for the line kernel's buffers beside the others, it starts on
+ * the tile kernel (the voxels of one tile on the TMEM lanes);
+ * b200bsp_autotune may move it to the x-lane kernel (voxel x on the lanes,
+ * 3 <= vox_per_rgn[1] <= 10) and back, and image ROIs (b200bsp_set_roi) move
+ * it to the x-lane kernel.  XLANE and TILE pin one of the tensor-core kernels
  * (XLANE on a grid it cannot take is B200BSP_E_UNSUPPORTED; with TILE
  * pinned, image ROIs are B200BSP_E_UNSUPPORTED in the tensor-core form). */
 #define B200BSP_TC_KERNEL_AUTO   0
@@ -251,7 +252,9 @@ int b200bsp_set_wait_limit (b200bsp_ctx* ctx, int polls, int withhold_mma);
 
 /* Testing aid: the nth device allocation made by the next b200bsp_create
  * calls of this thread fails as if the device were full (0 disables).  The
- * create returns B200BSP_E_OOM and releases everything it allocated. */
+ * create returns B200BSP_E_OOM and releases everything it allocated; the
+ * last one, the line kernel's, leaves a context without that kernel
+ * (B200BSP_TC_KERNEL_AUTO), as on a device that lacks the room for it. */
 void b200bsp_debug_fail_alloc (int nth);
 
 /* Testing aid: nonzero makes this thread's b200bsp_optimize_lbfgs calls

@@ -244,7 +244,7 @@ eqsp_range (const float* d_img, size_t n, int bins, float* d_scratch,
 
 void
 mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
-    bool line, Arena& dev, Arena& pinned)
+    Arena& dev, Arena& pinned)
 {
     s->bins = bins;
     s->window = window;
@@ -258,9 +258,6 @@ mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
     }
     dev.add (&s->d_fbin, nf);
     dev.add (&s->d_mbin, nm);
-    if (line && window == B200BSP_MI_PVI8) {
-        dev.add (&s->d_mquad, nm * sizeof (uint32_t));
-    }
     dev.add (&s->d_hist, nh * sizeof (unsigned long long));
     dev.add (&s->d_histd, nh * sizeof (double));
     dev.add (&s->d_lut, bins * bins * sizeof (float));
@@ -271,6 +268,13 @@ mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
     dev.add (&s->d_count_part, g.ntiles * sizeof (int));
     pinned.add (&s->h_histd, nh * sizeof (double));
     pinned.add (&s->h_res, sizeof (DevResult));
+}
+
+void
+mi_alloc_line (MiState* s, const BspGeom& g, Arena& dev)
+{
+    const size_t nm = (size_t) g.mdim[0] * g.mdim[1] * g.mdim[2];
+    if (s->window == B200BSP_MI_PVI8) dev.add (&s->d_mquad, nm * sizeof (uint32_t));
 }
 
 int

@@ -49,9 +49,10 @@ struct MiState {
     DevResult* h_res = nullptr;
 };
 
-// Asks for the state's buffers (line: for the line kernel as well).
+// Asks for the state's buffers; then for those of the line kernel.
 void mi_alloc (MiState* s, const BspGeom& g, int bins, int window, int hist,
-    bool line, Arena& dev, Arena& pinned);
+    Arena& dev, Arena& pinned);
+void mi_alloc_line (MiState* s, const BspGeom& g, Arena& dev);
 int mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
     const float* d_moving, size_t nf, size_t nm, cudaStream_t st);
 // passes: MI_PASS_HIST (histograms into d_hist), MI_PASS_GRAD (score and

@@ -659,8 +659,6 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
             if (o.tc_kernel == B200BSP_TC_KERNEL_AUTO
                 && line_plan (g, &c->lplan, sm_count)) {
                 c->use_line = true;
-                alloc ((void**) &c->d_rows, line_row_elems (g, c->lplan)
-                    * sizeof (float));
                 score_parts = std::max (score_parts, (size_t) c->lplan.nblocks);
             }
         }
@@ -680,11 +678,27 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
     score_parts = std::max (score_parts, (size_t) std::max (c->nscore_parts, 1));
     alloc ((void**) &c->d_score_part, score_parts * sizeof (double));
     alloc ((void**) &c->d_count_part, score_parts * sizeof (int));
-    mi_alloc (&c->mi, c->geom, o.mi_bins, o.mi_window, o.mi_hist, c->use_line,
-        dev, pinned);
+    mi_alloc (&c->mi, c->geom, o.mi_bins, o.mi_window, o.mi_hist, dev, pinned);
     reg_alloc (&c->reg, c->geom, dev, pinned);
     if (!rc2) {
-        cudaError_t e = dev.take (false, &c->d_slab);
+        // The line kernel's buffers come last: where they do not fit beside
+        // the others the context does without that kernel.
+        const size_t common = dev.all.size ();
+        cudaError_t e = cudaErrorMemoryAllocation;
+        if (c->use_line) {
+            dev.add (&c->d_rows, line_row_elems (g, c->lplan) * sizeof (float));
+            mi_alloc_line (&c->mi, c->geom, dev);
+            const bool deny = g_fail_alloc > 0 && --g_fail_alloc == 0;
+            if (!deny) e = dev.take (false, &c->d_slab);
+            if (e != cudaSuccess) {
+                cudaGetLastError ();
+                dev.all.resize (common);
+                c->use_line = false;
+                c->d_rows = nullptr;
+                c->mi.d_mquad = nullptr;
+            }
+        }
+        if (!c->use_line) e = dev.take (false, &c->d_slab);
         if (e == cudaSuccess) e = pinned.take (true, &c->h_slab);
         if (e != cudaSuccess) {
             cudaGetLastError ();
