@@ -368,9 +368,9 @@ __device__ __forceinline__ void
 line_use (const LineArgs& a, int ly, const Vox& v,
     Row (&q)[4], float& scf, int& cnt)
 {
-    float diff = line_value (v) - v.fv;
-    diff = v.ok ? diff : 0.f;
-    scf = fmaf (diff, diff, scf);
+    const float diff = line_value (v) - v.fv;
+    const float in = v.ok ? diff : 0.f;
+    scf = fmaf (in, in, scf);
     cnt += v.ok ? 1 : 0;
     u64 cxy;
     float cz;
@@ -383,7 +383,9 @@ line_use (const LineArgs& a, int ly, const Vox& v,
         cxy = mul2 (pk (diff, diff), pk (gd[0], gd[1]));
         cz = diff * gd[2];
     }
-    line_adjoint<R> (a.wy[ly], cxy, cz, q);
+    // selected, not multiplied by 0: a voxel outside has read the moving
+    // image's border, which may hold infinities or NaN
+    line_adjoint<R> (a.wy[ly], v.ok ? cxy : 0ull, v.ok ? cz : 0.f, q);
 }
 
 // Parzen pass 2 at a loaded voxel: 1/(N delta_m) * sum over the window's
@@ -404,13 +406,14 @@ line_use_pz (const LineArgs& a, int ly, const Vox& v, const float* slut, float s
         + (s * fmaf (1.5f, s, -2.f)) * row[2] - (0.5f * f * f) * row[3];
     float gi[3];
     trilinear_igrad (v.w2, v.cr, v.clamp, gi);
-    const float sc = v.ok ? scale * sum : 0.f;
+    const float sc = scale * sum;
     const float* p = a.g.mproj;
     float dc[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
         dc[c] = AXIS ? sc * (p[4 * c] * gi[c])
                      : sc * (p[c] * gi[0] + p[3 + c] * gi[1] + p[6 + c] * gi[2]);
+        dc[c] = v.ok ? dc[c] : 0.f;         // (as in line_use)
     }
     line_adjoint<R> (a.wy[ly], pk (dc[0], dc[1]), dc[2], q);
 }

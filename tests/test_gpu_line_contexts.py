@@ -7,7 +7,7 @@ import oracle as O
 import plastimatch_b200 as P
 from conftest import rel_err
 from plastimatch_b200 import synth
-from plastimatch_b200.geometry import BsplineGrid
+from plastimatch_b200.geometry import BsplineGrid, Volume
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +48,34 @@ def test_without_room_for_its_buffers_a_context_keeps_the_tile_kernel():
             got, want = getattr(ctx, call)(coeff), getattr(tile, call)(coeff)
             assert got[0] == want[0] and got[2] == want[2] > 0
             np.testing.assert_array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("angle", [0.0, 10.0])
+@pytest.mark.parametrize("what", ["nearest", "trilinear", "parzen"])
+def test_voxels_outside_leave_no_nan(what, angle):
+    """A NaN in the moving image's first plane, which only voxels outside the
+    image read (at x = -0.6; the next ones, at 1.7 and beyond, read planes 1
+    and up), changes no bit of the results."""
+    a = np.deg2rad(angle)
+    dcos = (np.cos(a), -np.sin(a), 0.0, np.sin(a), np.cos(a), 0.0, 0.0, 0.0, 1.0)
+    f = synth.gaussian_blobs((16, 30, 20), spacing=(1, 1, 1), seed=5).img
+    m = synth.gaussian_blobs((40, 30, 20), spacing=(1, 1, 1), seed=6).img
+    fixed = Volume(f, origin=(0.0, 0.0, 0.0), spacing=(2.3, 1.0, 1.0), dcos=dcos)
+    # the moving image begins 0.6 mm along x behind the fixed one's origin
+    moving = Volume(m, origin=(0.6 * dcos[0], 0.6 * dcos[3], 0.0),
+                    spacing=(1.0, 1.0, 1.0), dcos=dcos)
+    grid = BsplineGrid.for_volume(fixed, (4, 5, 6))
+    coeff = synth.random_coeff(grid, 0.02, 7)
+    kw = (dict(mi_window="parzen") if what == "parzen" else dict(mse_grad=what))
+    out = []
+    with P.Context(fixed, moving, grid, **kw) as ctx:
+        assert ctx.mse_kernel()[0] == "line"
+        for border in (float(m.mean()), np.nan):
+            img = m.copy()
+            img[:, :, 0] = border
+            ctx.set_images(None, img)
+            out.append(ctx.score_mi(coeff) if what == "parzen"
+                       else ctx.score_mse(coeff))
+    (s0, g0, n0), (s1, g1, n1) = out
+    assert 0 < n0 == n1 < f.size and s0 == s1
+    np.testing.assert_array_equal(g0, g1)
