@@ -917,10 +917,15 @@ stage_up (b200bsp_ctx* c, const float* coeff)
 
 // The gradient in d_grad to host memory the same way, after everything else
 // on the stream (up to four parts, each waited for and copied out while the
-// next one is on its way); returns when the last one is there.
+// next one is on its way); returns when the last one is there.  Page-locked
+// memory takes the copy itself, which the caller waits for.
 static cudaError_t
 stage_down (b200bsp_ctx* c, float* grad)
 {
+    if (mapped_alias (grad)) {
+        return cudaMemcpyAsync (grad, c->d_grad, c->num_coeff * sizeof (float),
+            cudaMemcpyDeviceToHost, c->stream);
+    }
     const int64_t part = std::max<int64_t> (STAGE_PART, (c->num_coeff + 3) / 4);
     cudaError_t e = cudaSuccess;
     int k = 0;
