@@ -1978,8 +1978,11 @@ field_warp (b200bsp_ctx* c, const float* coeff, float* vf, float* warped,
         whole = whole && g.roi_off[d] == 0 && g.roi_dim[d] == g.fdim[d];
     }
     if (vf && !whole) CK (cudaMemsetAsync (target, 0, bytes, c->stream));
+    // (an FP32 context and one with a pinned kernel keep the 64-tap field)
     LinePlan p;
-    if (line_plan (g, &p, c->sm_count)) {
+    if (c->opts.form == B200BSP_FORM_TC
+        && c->opts.tc_kernel == B200BSP_TC_KERNEL_AUTO
+        && line_plan (g, &p, c->sm_count)) {
         CK (launch_field_line (g, p, dcoeff, c->d_luts, c->d_moving,
             default_value, vf ? target : nullptr, vf ? nullptr : target,
             c->stream));

@@ -125,3 +125,42 @@ def test_page_locked_gradients_are_copied_once(call):
         np.testing.assert_array_equal(hg.numpy(), dg.cpu().numpy())
     t_copy = best(lambda: hg.copy_(dg, non_blocking=True))
     assert t_host - t_dev < 1.5 * t_copy + 40e-6, (t_dev, t_host, t_copy)
+
+
+def _field_64_taps(grid, coeff):
+    """The field as the plain kernel sums it: float weights ((z y) x), one
+    fused multiply-add a knot, x fastest (double products are exact, so that
+    each sum is rounded to float once, up to the rare double rounding)."""
+    f4 = np.float32
+    nx, ny, nz = grid.roi_dim
+    lut = [O.port_basis_lut(v).reshape(v, 4).astype(f4) for v in grid.vox_per_rgn]
+    c = coeff.reshape(grid.cdims[2], grid.cdims[1], grid.cdims[0], 3)
+    at = [np.arange(n) // v for n, v in zip((nx, ny, nz), grid.vox_per_rgn)]
+    w = [t[np.arange(n) % v] for t, n, v in zip(lut, (nx, ny, nz), grid.vox_per_rgn)]
+    d = np.zeros((nz, ny, nx, 3), f4)
+    for k in range(4):
+        for j in range(4):
+            b = w[1][:, j][None, :] * w[2][:, k][:, None]
+            for i in range(4):
+                a = w[0][:, i][None, None, :] * b[:, :, None]
+                t = c[at[2] + k][:, at[1] + j][:, :, at[0] + i]
+                d = (a[..., None].astype(np.float64) * t + d).astype(f4)
+    return d
+
+
+@pytest.mark.parametrize("kw", [dict(form="fp32"), dict(tc_kernel="tile"),
+                                dict(tc_kernel="xlane")])
+def test_field_of_a_pinned_context_keeps_its_kernel(kw):
+    """The field of an FP32 context, and of one with a pinned tensor-core
+    kernel, on a grid that the line kernel takes: the plain kernel's 64
+    products a voxel, bit for bit (but for double roundings, 1e-4 of the
+    values at most), and the warp that goes with it."""
+    fixed, moving, grid, coeff = _case()
+    want = _field_64_taps(grid, coeff)
+    with P.Context(fixed, moving, grid, **kw) as ctx:
+        ctx.set_images()
+        vf = ctx.interpolate_vf(coeff)
+        w = ctx.warp(coeff, -7.0)
+    assert (vf != want).mean() <= 1e-4, (vf != want).mean()
+    ref = synth.warp_trilinear(moving, fixed, grid, coeff, -7.0).img
+    assert (np.abs(w - ref) > 0.1).mean() < 1e-4
