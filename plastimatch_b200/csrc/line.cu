@@ -96,7 +96,7 @@ struct LineArgs {
     const float* nvf;    //   [1]: 1 / (N delta_m)
     u64* hist;           // pass 1: f[B], m[B], j[B * B], count
     int bins;
-    float pz_min, pz_inv;                   // moving value -> window centre
+    float pz_min, pz_delta, pz_inv;         // moving value -> window centre
     float* out;          // field (xyz per voxel) or warped image
     float outside;
     bool roi_same;       // the moving ROI is a mask on the moving image's grid
@@ -388,6 +388,13 @@ line_use (const LineArgs& a, int ly, const Vox& v,
     line_adjoint<R> (a.wy[ly], v.ok ? cxy : 0ull, v.ok ? cz : 0.f, q);
 }
 
+// The Parzen window's centre at a loaded voxel (parzen_centre's value).
+__device__ __forceinline__ float
+line_pz_centre (const LineArgs& a, const Vox& v)
+{
+    return line_quotient (line_value (v) - a.pz_min, a.pz_delta, a.pz_inv) + 2.f;
+}
+
 // Parzen pass 2 at a loaded voxel: 1/(N delta_m) * sum over the window's
 // bins of beta3'(k - u) log(p(f, k) / p_m(k)) (slut, shared memory), times
 // the world gradient of the trilinear interpolant (proj^T times the index
@@ -398,7 +405,7 @@ template <bool AXIS, int R>
 __device__ __forceinline__ void
 line_use_pz (const LineArgs& a, int ly, const Vox& v, const float* slut, float scale, Row (&q)[4])
 {
-    const float u = fmaf (line_value (v) - a.pz_min, a.pz_inv, 2.f);
+    const float u = line_pz_centre (a, v);
     const int k0 = parzen_first_bin (u, a.bins);
     const float f = u - (float) (k0 + 1), s = 1.f - f;
     const float* row = slut + v.fb * a.bins + k0;
@@ -456,7 +463,7 @@ __device__ __forceinline__ void
 line_use_pz_hist (const LineArgs& a, const Vox& v, uint32_t* sh, Run& r)
 {
     if (!v.ok) return;
-    const float u = fmaf (line_value (v) - a.pz_min, a.pz_inv, 2.f);
+    const float u = line_pz_centre (a, v);
     const int k0 = parzen_first_bin (u, a.bins);
     const float f = u - (float) (k0 + 1), s = 1.f - f;
     const float f2 = f * f, s2 = s * s;
@@ -1269,6 +1276,7 @@ launch_mi_line (const BspGeom& g, const LinePlan& p, bool hist_pass,
     a.hist = mi.hist;
     a.mimg = mi.mimg;
     a.pz_min = mi.m_min;
+    a.pz_delta = mi.m_delta;
     a.pz_inv = 1.f / mi.m_delta;
     a.rows = rows;
     if (!mi.parzen) {

@@ -1,5 +1,7 @@
-// Index arithmetic of the line kernel, for the device and for the host.
+// Arithmetic of the line kernel that the host shares.
 #pragma once
+
+#include <cmath>
 
 #ifdef __CUDACC__
 #define LINE_FN __host__ __device__ __forceinline__
@@ -27,6 +29,16 @@ line_corner (const int bits[3], int nx, int ny, unsigned corner0)
 {
     return (unsigned) bits[0] + (unsigned) nx * ((unsigned) bits[1]
         + (unsigned) ny * (unsigned) bits[2]) + corner0;
+}
+
+// x / d, rounded correctly, with inv the rounded 1 / d: the quotient's exact
+// remainder once more (Markstein's theorem, IBM J. Res. Dev. 34(1), 1990).
+// d and inv are normal numbers.
+LINE_FN float
+line_quotient (float x, float d, float inv)
+{
+    const float q = x * inv;
+    return fmaf (fmaf (-q, d, x), inv, q);
 }
 
 }  // namespace b200

@@ -1270,7 +1270,9 @@ mi_passes_on (b200bsp_ctx* c, const BspGeom& g, const float* dcoeff,
     // its pass 2 stays with the field it has always been formed from.
     if (line_now (c) && !roi) {
         const bool parzen = c->opts.mi_window == B200BSP_MI_PARZEN;
-        const int now = parzen ? passes : passes & MI_PASS_HIST;
+        int now = parzen ? passes : passes & MI_PASS_HIST;
+        // (its window centres multiply by the bin width's reciprocal)
+        if (parzen && !std::isnormal (1.f / c->mi.pz_mdelta)) now = 0;
         LinePlan p = c->lplan;
         bool ok = now != 0;
         if (ok && &g != &c->geom) ok = line_plan (g, &p, c->sm_count);

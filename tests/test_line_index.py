@@ -1,6 +1,7 @@
-"""The line kernel's corner index (line_index.cuh) on the host, with signed
-overflow trapping: for every image it takes, the smallest and the largest
-included, the corners' indices are those of 64-bit arithmetic."""
+"""The line kernel's arithmetic that the host shares (line_index.cuh), with
+signed overflow trapping: for every image it takes, the smallest and the
+largest included, the corners' indices are those of 64-bit arithmetic; a
+quotient by a multiplication is the division's, bit for bit."""
 import os
 import shutil
 import subprocess
@@ -44,19 +45,51 @@ int main (int argc, char** argv)
 """
 
 
-@pytest.fixture(scope="module")
-def program(tmp_path_factory):
+QUOTIENT = r"""
+#include <cstdint>
+#include "line_index.cuh"
+using namespace b200;
+
+int main ()
+{
+    uint64_t r = 88172645463325252ull;
+    auto uniform = [&] {
+        r ^= r << 13; r ^= r >> 7; r ^= r << 17;
+        return (float) (r >> 40) / 16777216.f;
+    };
+    // image ranges of 2^-20 to 2^30 grey levels, 5 to 64 bins
+    for (int t = 0; t < 2000; t++) {
+        const float range = std::exp2 (-20.f + 50.f * uniform ());
+        const float d = range / (float) (1 + (int) (60.f * uniform ()));
+        for (int k = 0; k < 1000; k++) {
+            const float x = range * uniform ();
+            volatile float want = x / d;
+            if (line_quotient (x, d, 1.f / d) != want) return 1;
+        }
+    }
+    return 0;
+}
+"""
+
+
+def _build(tmp_path_factory, name, text):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no host compiler")
-    d = tmp_path_factory.mktemp("line_index")
-    src, exe = d / "index.cpp", d / "index"
-    src.write_text(PROGRAM)
-    subprocess.run([cxx, "-std=c++17", "-O1", "-fsanitize=undefined",
+    d = tmp_path_factory.mktemp(name)
+    src, exe = d / "main.cpp", d / "main"
+    src.write_text(text)
+    subprocess.run([cxx, "-std=c++17", "-O1", "-ffp-contract=off",
+                    "-fsanitize=undefined",
                     "-fsanitize-undefined-trap-on-error", "-x", "c++", "-I",
                     os.path.join(ROOT, "plastimatch_b200", "csrc"), str(src),
                     "-o", str(exe)], check=True)
     return str(exe)
+
+
+@pytest.fixture(scope="module")
+def program(tmp_path_factory):
+    return _build(tmp_path_factory, "index", PROGRAM)
 
 
 @pytest.mark.parametrize("dim", [(2, 2, 2), (3, 2, 5), (64, 64, 64),
@@ -64,3 +97,8 @@ def program(tmp_path_factory):
                                  (1023, 1025, 1024), (1 << 22, 2, 127)])
 def test_corner_index(program, dim):
     assert subprocess.run([program] + [str(v) for v in dim]).returncode == 0
+
+
+def test_quotient(tmp_path_factory):
+    exe = _build(tmp_path_factory, "quotient", QUOTIENT)
+    assert subprocess.run([exe]).returncode == 0
