@@ -164,21 +164,3 @@ def test_field_of_a_pinned_context_keeps_its_kernel(kw):
     assert (vf != want).mean() <= 1e-4, (vf != want).mean()
     ref = synth.warp_trilinear(moving, fixed, grid, coeff, -7.0).img
     assert (np.abs(w - ref) > 0.1).mean() < 1e-4
-
-
-@pytest.mark.parametrize("bins", [5, 20, 32, 64])
-def test_parzen_centres_are_the_plain_forms(bins):
-    """Without a displacement every voxel samples a moving voxel exactly, so
-    the window centre alone decides the weights: the histograms are the FP32
-    form's, every integer of them."""
-    fixed = synth.gaussian_blobs((40, 36, 32), spacing=(1, 1, 1), seed=9)
-    moving = synth.gaussian_blobs((41, 37, 33), spacing=(1, 1, 1), seed=10)
-    grid = BsplineGrid.for_volume(fixed, (4, 5, 6))
-    h = []
-    for form in ("fp32", "tc"):
-        with P.Context(fixed, moving, grid, form=form, mi_window="parzen",
-                       mi_bins=bins) as ctx:
-            ctx.set_images()
-            h.append(ctx.mi_hist(np.zeros(grid.num_coeff, np.float32)))
-    assert h[0][-1] == fixed.img.size
-    np.testing.assert_array_equal(h[1], h[0])
