@@ -85,10 +85,12 @@ struct b200bsp_ctx {
     unsigned wait_limit = XL_DEFAULT_WAIT_LIMIT;
     int withhold_mma = 0;     // b200bsp_set_wait_limit's testing aid
     // the line kernel (line.cu), an AUTO context's choice on the grids that
-    // line_plan takes
+    // line_plan takes (line_grid; use_line with its buffers)
+    bool line_grid = false;
     bool use_line = false;
     int line_hold = 0;        // > 0 inside the optimiser and the autotuner
     LinePlan lplan;
+    LinePlan wplan;           // PVI-8 pass 1 over the whole image
     float* d_rows = nullptr;
     // b200bsp_score's device path: the regulariser on a second stream,
     // overlapping the tile kernel, its gradient kept in double
@@ -300,6 +302,9 @@ check_volume (const b200bsp_volume* v, const char* what)
     }
     return B200BSP_OK;
 }
+
+static int mi_whole_image_pass1 (const b200bsp_ctx* c);
+static BspGeom mi_whole_image (const b200bsp_ctx* c);
 
 static void
 free_all (b200bsp_ctx* c)
@@ -658,7 +663,11 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
             }
             if (o.tc_kernel == B200BSP_TC_KERNEL_AUTO
                 && line_plan (g, &c->lplan, sm_count)) {
-                c->use_line = true;
+                c->line_grid = c->use_line = true;
+                if (mi_whole_image_pass1 (c) == 1) {
+                    const BspGeom g1 = mi_whole_image (c);
+                    c->use_line = line_plan (g1, &c->wplan, sm_count);
+                }
                 score_parts = std::max (score_parts, (size_t) c->lplan.nblocks);
             }
         }
@@ -1258,6 +1267,15 @@ b200bsp_mse_kernel (const b200bsp_ctx* c, int* kernel, int* tiles,
     return B200BSP_OK;
 }
 
+// The geometry of pass 1 over the whole image.
+static BspGeom
+mi_whole_image (const b200bsp_ctx* c)
+{
+    BspGeom g = c->geom;
+    for (int d = 0; d < 3; d++) g.roi_dim[d] = g.fdim[d];
+    return g;
+}
+
 // One or both MI passes on the context's form (tensor-core modes where they
 // apply); gradients to grad (float) or grad64 (double), device pointers.
 static int
@@ -1273,11 +1291,9 @@ mi_passes_on (b200bsp_ctx* c, const BspGeom& g, const float* dcoeff,
         int now = parzen ? passes : passes & MI_PASS_HIST;
         // (its window centres multiply by the bin width's reciprocal)
         if (parzen && !std::isnormal (1.f / c->mi.pz_mdelta)) now = 0;
-        LinePlan p = c->lplan;
-        bool ok = now != 0;
-        if (ok && &g != &c->geom) ok = line_plan (g, &p, c->sm_count);
-        if (ok) {
-            const int rc = mi_run_line (&c->mi, g, p, c->d_rows, dcoeff,
+        if (now) {
+            const int rc = mi_run_line (&c->mi, g,
+                &g == &c->geom ? c->lplan : c->wplan, c->d_rows, dcoeff,
                 c->d_moving, c->d_luts, c->d_res, grad, grad64, c->stream,
                 &c->last_launches, now);
             passes &= ~now;
@@ -1338,8 +1354,7 @@ mi_passes (b200bsp_ctx* c, const float* dcoeff, float* grad, double* grad64,
         && mi_whole_image_pass1 (c) == 1) {
         // pass 1 over the whole image with the same tile grid, pass 2
         // over the ROI
-        BspGeom g1 = c->geom;
-        for (int d = 0; d < 3; d++) g1.roi_dim[d] = g1.fdim[d];
+        const BspGeom g1 = mi_whole_image (c);
         int rc = mi_passes_on (c, g1, dcoeff, grad, grad64, MI_PASS_HIST);
         if (rc || !(passes & MI_PASS_GRAD)) return rc;
         passes = MI_PASS_GRAD;
@@ -1981,11 +1996,8 @@ field_warp (b200bsp_ctx* c, const float* coeff, float* vf, float* warped,
     }
     if (vf && !whole) CK (cudaMemsetAsync (target, 0, bytes, c->stream));
     // (an FP32 context and one with a pinned kernel keep the 64-tap field)
-    LinePlan p;
-    if (c->opts.form == B200BSP_FORM_TC
-        && c->opts.tc_kernel == B200BSP_TC_KERNEL_AUTO
-        && line_plan (g, &p, c->sm_count)) {
-        CK (launch_field_line (g, p, dcoeff, c->d_luts, c->d_moving,
+    if (c->line_grid) {
+        CK (launch_field_line (g, c->lplan, dcoeff, c->d_luts, c->d_moving,
             default_value, vf ? target : nullptr, vf ? nullptr : target,
             c->stream));
     } else {
