@@ -1304,17 +1304,22 @@ launch_field_line (const BspGeom& g, const LinePlan& p, const float* coeff,
 }
 
 // Bins of the 2 x 2 moving voxels from each voxel on (x fastest, a byte
-// each): one 4-byte load in place of four of one byte.
+// each): one 4-byte load in place of four of one byte.  A warp takes a row:
+// bound by memory, 5 bytes a voxel.
 __global__ void
-bin_quad_kernel (int nx, int ny, long long n, const uint8_t* __restrict__ bin,
+bin_quad_kernel (int nx, int ny, long long rows, const uint8_t* __restrict__ bin,
     uint32_t* __restrict__ quad)
 {
-    for (long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long) gridDim.x * blockDim.x) {
-        const int x = (int) (i % nx), y = (int) ((i / nx) % ny);
-        const int dx = x + 1 < nx ? 1 : 0, dy = y + 1 < ny ? nx : 0;
-        quad[i] = bin[i] | (uint32_t) bin[i + dx] << 8
-            | (uint32_t) bin[i + dy] << 16 | (uint32_t) bin[i + dy + dx] << 24;
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    for (long long r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+         r < rows; r += nw) {
+        const uint8_t* b = bin + r * nx;
+        const int dy = r % ny + 1 < ny ? nx : 0;
+        for (int x = threadIdx.x & 31; x < nx; x += 32) {
+            const int dx = x + 1 < nx ? 1 : 0;
+            quad[r * nx + x] = b[x] | (uint32_t) b[x + dx] << 8
+                | (uint32_t) b[x + dy] << 16 | (uint32_t) b[x + dy + dx] << 24;
+        }
     }
 }
 
@@ -1323,7 +1328,7 @@ launch_bin_quad (const int dim[3], const uint8_t* bin, uint32_t* quad,
     cudaStream_t st)
 {
     bin_quad_kernel<<<1184, 256, 0, st>>> (dim[0], dim[1],
-        (long long) dim[0] * dim[1] * dim[2], bin, quad);
+        (long long) dim[1] * dim[2], bin, quad);
     return cudaGetLastError ();
 }
 

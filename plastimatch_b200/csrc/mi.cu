@@ -281,6 +281,7 @@ int
 mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
     const float* d_moving, size_t nf, size_t nm, cudaStream_t st)
 {
+    s->quads = false;
     if (s->window == B200BSP_MI_PARZEN) {
         // value ranges mapped onto bins 2 .. bins - 2 (two padding bins at
         // either end hold the cubic window's tails)
@@ -303,10 +304,6 @@ mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
             s->d_fkey, s->d_fbin, st);
         if (!rc) rc = vopt_bins (d_moving, nm, s->bins, &s->m_offset,
             &s->m_delta, s->d_mkey, s->d_mbin, st);
-        if (!rc && s->d_mquad && launch_bin_quad (g.mdim, s->d_mbin,
-                s->d_mquad, st) != cudaSuccess) {
-            rc = B200BSP_E_CUDA;
-        }
         if (rc) return rc;
         s->ready = true;
         return B200BSP_OK;
@@ -321,7 +318,6 @@ mi_set_images (MiState* s, const BspGeom& g, const float* d_fixed,
         s->f_offset, s->f_delta, s->bins, s->d_fbin);
     bin_image_kernel<<<1184, 256, 0, st>>> (d_moving, (long long) nm,
         s->m_offset, s->m_delta, s->bins, s->d_mbin);
-    if (s->d_mquad) launch_bin_quad (g.mdim, s->d_mbin, s->d_mquad, st);
     if (cudaGetLastError () != cudaSuccess) return B200BSP_E_CUDA;
     s->ready = true;
     return B200BSP_OK;
@@ -1013,6 +1009,23 @@ mi_run_line (MiState* s, const BspGeom& g, const LinePlan& plan,
     mi.m_min = s->pz_mmin;
     mi.m_delta = s->pz_mdelta;
     if (passes & MI_PASS_HIST) {
+        // The quads of new images: formed by the first pass that reads them,
+        // so that contexts that evaluate no MI do not pay for them.  A graph that is
+        // being captured forms its own each time, since the images may
+        // change between its launches.
+        if (s->d_mquad) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing (st, &cap) != cudaSuccess) {
+                return B200BSP_E_CUDA;
+            }
+            const bool captured = cap != cudaStreamCaptureStatusNone;
+            if (captured || !s->quads) {
+                if (launch_bin_quad (g.mdim, s->d_mbin, s->d_mquad, st)
+                    != cudaSuccess) return B200BSP_E_CUDA;
+                s->quads = !captured;
+                if (launches) *launches += 1;
+            }
+        }
         if (cudaMemsetAsync (s->d_hist, 0, (nh + 1) * sizeof (unsigned long long),
                 st) != cudaSuccess
             || launch_mi_line (g, plan, true, mi, d_coeff, d_luts, nullptr, st)

@@ -36,6 +36,7 @@ struct MiState {
     uint8_t* d_fbin = nullptr;                // fixed-image bin per voxel
     uint8_t* d_mbin = nullptr;                // moving-image bin per voxel
     uint32_t* d_mquad = nullptr;              // line kernel: bins of 2 x 2 voxels
+    bool quads = false;                       //   formed from d_mbin
     unsigned long long* d_hist = nullptr;     // f[B], m[B], j[B*B], N (fixed point)
     double* d_histd = nullptr;                // f, m, j as doubles
     float* d_lut = nullptr;                   // dS/dP per joint bin (0 = skip)

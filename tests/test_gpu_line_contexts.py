@@ -220,3 +220,75 @@ def test_histograms_of_noise_take_no_longer(bins):
                 best = min(best, time.perf_counter() - t0)
             t.append(best)
     assert t[1] < 1.1 * t[0], t
+
+
+def _mi_device(ctx, coeff, out):
+    """b200bsp_score (MI) with device outputs, stream-ordered."""
+    import ctypes as C
+    rc = P.lib().b200bsp_score(
+        ctx._h, coeff.data_ptr(), 1, C.c_float(1.0), None, out[0].data_ptr(),
+        out[1].data_ptr(), None, out[2].data_ptr())
+    assert rc == 0
+
+
+def test_new_images_reach_pass_1():
+    """PVI-8's pass 1 reads an image of the moving bins that its first
+    evaluation forms: after b200bsp_set_images it is the new one, in direct
+    calls and in a graph captured before."""
+    import torch
+    fixed, moving, grid, coeff = _case()
+    other = synth.gaussian_blobs(moving.dim, spacing=moving.spacing, seed=77)
+    with P.Context(fixed, other, grid) as ctx:
+        ctx.set_images()
+        s_new, g_new, n_new = ctx.score_mi(coeff)
+    dc = torch.from_numpy(coeff).cuda()
+
+    def outputs():
+        return (torch.zeros(1, device="cuda"), torch.zeros_like(dc),
+                torch.zeros(1, dtype=torch.int64, device="cuda"))
+    stream = torch.cuda.Stream()
+    for evaluate_first in (False, True):
+        with P.Context(fixed, moving, grid) as ctx:
+            ctx.set_stream(stream.cuda_stream)
+            ctx.set_images()
+            if evaluate_first:
+                s_old = ctx.score_mi(coeff)[0]
+                assert s_old != s_new
+            out, graph = outputs(), torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph, stream=stream,
+                                  capture_error_mode="relaxed"):
+                _mi_device(ctx, dc, out)
+            ctx.set_images(None, other.img)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert out[0].item() == s_new and out[2].item() == n_new
+            np.testing.assert_array_equal(out[1].cpu().numpy(), g_new)
+            s, g, n = ctx.score_mi(coeff)
+            assert s == s_new and n == n_new
+            np.testing.assert_array_equal(g, g_new)
+            del graph
+
+
+def test_images_of_an_mse_context_cost_what_they_did():
+    """b200bsp_set_images does nothing for the line kernel that a context
+    pinned to the tile kernel does without (12 % of its time, when it formed
+    pass 1's image of the moving bins)."""
+    import time
+
+    import torch
+    fixed = synth.gaussian_blobs((256, 256, 96), seed=3)
+    grid = BsplineGrid.for_volume(fixed, 8)
+    img = torch.from_numpy(fixed.img).cuda()
+    best = {}
+    for _ in range(2):
+        for kernel in ("tile", "auto"):
+            with P.Context(fixed, fixed, grid, tc_kernel=kernel) as ctx:
+                for _ in range(40):
+                    torch.cuda.synchronize()
+                    t0 = time.perf_counter()
+                    ctx.set_images(img, img)
+                    torch.cuda.synchronize()
+                    best[kernel] = min(best.get(kernel, np.inf),
+                                       time.perf_counter() - t0)
+    assert best["auto"] < 1.06 * best["tile"], best
