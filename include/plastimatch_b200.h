@@ -326,9 +326,10 @@ int b200bsp_mse_kernel (const b200bsp_ctx* ctx, int* kernel, int* tiles,
  * src/base/bspline_interpolate.cxx:112-142): vf is dim[0]*dim[1]*dim[2]*3
  * floats of the fixed image, xyz interleaved; voxels outside the ROI are
  * zero.  A tensor-core-form context with the AUTO kernel takes the line
- * kernel's separable sums on the grids of that kernel; the FP32 form, a
- * pinned kernel and other grids take the 64 products a voxel one by one
- * (so does b200bsp_warp).  coeff and vf may be host or device memory; with a host vf the
+ * kernel's separable sums on the grids of that kernel (from 40000 voxels
+ * on); the FP32 form, a pinned kernel and other grids take the 64 products a
+ * voxel one by one (so does b200bsp_warp).  coeff and vf may be host or
+ * device memory; with a host vf the
  * first call allocates a device staging buffer of 12 bytes per fixed voxel,
  * kept until b200bsp_destroy. */
 int b200bsp_interpolate_vf (b200bsp_ctx* ctx, const float* coeff, float* vf);

@@ -1995,8 +1995,14 @@ field_warp (b200bsp_ctx* c, const float* coeff, float* vf, float* warped,
         whole = whole && g.roi_off[d] == 0 && g.roi_dim[d] == g.fdim[d];
     }
     if (vf && !whole) CK (cudaMemsetAsync (target, 0, bytes, c->stream));
-    // (an FP32 context and one with a pinned kernel keep the 64-tap field)
-    if (c->line_grid) {
+    // An FP32 context and one with a pinned kernel keep the 64-tap field, as
+    // do images of some 35 voxels a side, where the launches are what counts
+    // and the line kernel's larger arguments cost a microsecond (calls one
+    // after another, field and warp: 24^3 4.9 and 5.1 us against 6.1 and 6.5,
+    // 33^3 4.9 and 6.2 against 6.1 and 6.6; 40^3 8.3 and 6.3 against 4.8 and
+    // 6.3).
+    const long long nroi = (long long) g.roi_dim[0] * g.roi_dim[1] * g.roi_dim[2];
+    if (c->line_grid && nroi >= 40000) {
         CK (launch_field_line (g, c->lplan, dcoeff, c->d_luts, c->d_moving,
             default_value, vf ? target : nullptr, vf ? nullptr : target,
             c->stream));

@@ -148,14 +148,16 @@ def _field_64_taps(grid, coeff):
     return d
 
 
-@pytest.mark.parametrize("kw", [dict(form="fp32"), dict(tc_kernel="tile"),
-                                dict(tc_kernel="xlane")])
-def test_field_of_a_pinned_context_keeps_its_kernel(kw):
+@pytest.mark.parametrize("dim,kw", [
+    ((48, 40, 36), dict(form="fp32")), ((48, 40, 36), dict(tc_kernel="tile")),
+    ((48, 40, 36), dict(tc_kernel="xlane")), ((34, 34, 34), dict())])
+def test_field_of_a_pinned_context_keeps_its_kernel(dim, kw):
     """The field of an FP32 context, and of one with a pinned tensor-core
-    kernel, on a grid that the line kernel takes: the plain kernel's 64
-    products a voxel, bit for bit (but for double roundings, 1e-4 of the
-    values at most), and the warp that goes with it."""
-    fixed, moving, grid, coeff = _case()
+    kernel, on a grid that the line kernel takes, and of a small image: the
+    plain kernel's 64 products a voxel, bit for bit (but for double
+    roundings, 1e-4 of the values at most), and the warp that goes with
+    it."""
+    fixed, moving, grid, coeff = _case(dim)
     want = _field_64_taps(grid, coeff)
     with P.Context(fixed, moving, grid, **kw) as ctx:
         ctx.set_images()
