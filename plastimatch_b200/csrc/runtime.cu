@@ -587,7 +587,10 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
     };
     alloc ((void**) &c->d_fixed, nf * sizeof (float));
     alloc ((void**) &c->d_moving, nm * sizeof (float));
-    if (o.mse_grad == 0) alloc ((void**) &c->d_mgrad, 3 * nm * sizeof (float));
+    // (a triple of zeros behind the last voxel's, for the line kernel)
+    if (o.mse_grad == 0) {
+        alloc ((void**) &c->d_mgrad, 3 * (nm + 1) * sizeof (float));
+    }
     int sm_count = 148;
     cudaDeviceGetAttribute (&sm_count, cudaDevAttrMultiProcessorCount, o.device);
     c->sm_count = sm_count;
@@ -782,6 +785,7 @@ b200bsp_create (const b200bsp_volume* fixed, const b200bsp_volume* moving,
         cudaMemcpyHostToDevice);
     cudaMemcpy (c->d_inv_dc, minv, 9 * sizeof (float), cudaMemcpyHostToDevice);
     cudaMemset (c->d_err, 0, sizeof (int));
+    if (c->d_mgrad) cudaMemset (c->d_mgrad + 3 * nm, 0, 3 * sizeof (float));
     if (c->use_line) {
         cudaMemset (c->d_rows, 0, line_row_elems (g, c->lplan) * sizeof (float));
     }
