@@ -872,7 +872,7 @@ line_kernel (const __grid_constant__ LineArgs a)
 // rows, counts and scores are written during this kernel's lifetime then:
 // they are read through L2, never as read-only data.
 
-constexpr int LF_MAX_THREADS = 512;
+constexpr int LF_MAX_THREADS = LINE_SPLIT_THREADS;
 
 struct LineFinishArgs {
     BspGeom g;
@@ -1169,6 +1169,7 @@ line_plan (const BspGeom& g, LinePlan* p, int sm_count)
         p->smem = m.total;
     }
     p->threads = 32 * p->nw;
+    p->sms = sm_count;
     basis_lut (p->wy, g.vpr[1]);
     p->nblocks = p->gpr * p->nys * g.rdims[2];
     return p->nys < 65536 && g.rdims[2] < 65536 && p->smem <= 200 * 1024;
@@ -1370,41 +1371,10 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     a.nys = p.nys;
     a.j = p.j;
     a.nxs = p.nxs;
-    // the whole row along x where it fits a block, else even parts
-    const int most = (2 * LF_MAX_THREADS - 2) / g.vpr[0] - 3;
-    const int nbx = (g.cdims[0] + most - 1) / most;
-    a.kxc = (g.cdims[0] + nbx - 1) / nbx;
-    const int threads = (((a.kxc + 3) * g.vpr[0] + 2) / 2 + 31) / 32 * 32;
-    // Knots along z a block, and parts its tiles' planes are split over: of
-    // the splits whose blocks are all resident at once (512 threads of 128
-    // registers an SM) the one with the shortest march, a block's own tile
-    // rows and the 3 beyond them times a latency and its planes.  Against 2
-    // to 8 knots and 1 to 4 parts by the number of blocks alone (some 300),
-    // the call takes at 131x117x83 vpr 6 25.7 us where that took 27.1, at
-    // 200x180x90 vpr 7x7x4 with ROIs 48.3 (51.5: 377 blocks of which 296
-    // were resident), eight uneven images 308 (317).  Where no split is
-    // resident (512x512x160) the row of 8 knots reads least: 343 us, 347
-    // with 5, 356 with 2; two blocks an SM in 96 registers, one in 128: 352.
-    double best = 0.0;
-    int parts = 0;
-    for (int kzc = 1; kzc <= 8; kzc++) {
-        const int n = nbx * g.cdims[1] * ((g.cdims[2] + kzc - 1) / kzc);
-        for (int p = 1; p <= std::min (g.vpr[2], 8); p++) {
-            if (p * threads > LF_MAX_THREADS
-                || n > 148 * (LF_MAX_THREADS / (p * threads))) break;
-            const double cost = (kzc + 3)
-                * (0.6 + 0.2 * ((g.vpr[2] + p - 1) / p));
-            if (parts && cost >= best) continue;
-            best = cost;
-            parts = p;
-            a.kzc = kzc;
-        }
-    }
-    const bool waves = parts == 0;
-    if (waves) {
-        a.kzc = 8;
-        parts = 1;
-    }
+    const LineSplit f = line_finish_split (g.cdims, g.vpr, p.sms);
+    const int threads = f.threads, parts = f.parts, nbx = f.nbx;
+    a.kxc = f.kxc;
+    a.kzc = f.kzc;
     const dim3 grid (nbx, g.cdims[1], (g.cdims[2] + a.kzc - 1) / a.kzc);
     const size_t smem = (size_t) 6 * a.kzc * threads * parts * sizeof (float);
     // the fewest rounds of at most five planes, evenly filled
@@ -1412,7 +1382,7 @@ launch_line_finish (const BspGeom& g, const LinePlan& p, const float* rows,
     const int rounds = (nz + 4) / 5;
     const int most_nz = (nz + rounds - 1) / rounds;
     auto k = line_finish_kernel<5, 1>;
-    if (waves && threads <= 320 && most_nz <= 4) k = line_finish_kernel<4, 2>;
+    if (f.waves && threads <= 320 && most_nz <= 4) k = line_finish_kernel<4, 2>;
     else if (most_nz <= 3) k = line_finish_kernel<3, 1>;
     else if (most_nz == 4) k = line_finish_kernel<4, 1>;
     if (smem > LN_PLAIN_SMEM) {

@@ -17,6 +17,7 @@ struct LinePlan {
                          // one's voxels beyond the ROI stay zero)
     int nblocks;
     int threads;
+    int sms;             // of the device
     size_t smem;
     float wy[40];        // y basis table (vpr[1] * 4)
 };

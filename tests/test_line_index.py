@@ -1,7 +1,9 @@
 """The line kernel's arithmetic that the host shares (line_index.cuh), with
 signed overflow trapping: for every image it takes, the smallest and the
-largest included, the corners' indices are those of 64-bit arithmetic; a
-quotient by a multiplication is the division's, bit for bit."""
+largest included, the corners' indices are those of 64-bit arithmetic; a quotient by
+a multiplication is the division's, bit for bit; the blocks of the rows'
+contraction are resident at once where the split says so, whatever the
+device's number of SMs."""
 import os
 import shutil
 import subprocess
@@ -71,6 +73,32 @@ int main ()
 }
 """
 
+SPLIT = r"""
+#include <initializer_list>
+#include "line_index.cuh"
+using namespace b200;
+
+int main ()
+{
+    const int sizes[] = {4, 7, 14, 23, 40, 55, 108, 160};
+    int resident = 0, waves = 0;
+    for (int sms : {20, 74, 132, 148, 160})
+    for (int vx : {3, 5, 8, 10}) for (int vz : {3, 5, 8, 10})
+    for (int cx : sizes) for (int cy : sizes) for (int cz : sizes) {
+        const int c[3] = {cx, cy, cz}, v[3] = {vx, 5, vz};
+        const LineSplit f = line_finish_split (c, v, sms);
+        const int block = f.threads * f.parts;
+        if (f.kxc * f.nbx < cx || f.kzc < 1 || f.kzc > 8 || f.parts > vz) return 1;
+        if (2 * f.threads < (f.kxc + 3) * vx + 1 || f.threads % 32) return 2;
+        if (block > LINE_SPLIT_THREADS) return 3;
+        const int n = f.nbx * cy * ((cz + f.kzc - 1) / f.kzc);
+        if (!f.waves && n > sms * (LINE_SPLIT_THREADS / block)) return 4;
+        (f.waves ? waves : resident)++;
+    }
+    return resident > 1000 && waves > 1000 ? 0 : 5;
+}
+"""
+
 
 def _build(tmp_path_factory, name, text):
     cxx = shutil.which("g++")
@@ -101,4 +129,9 @@ def test_corner_index(program, dim):
 
 def test_quotient(tmp_path_factory):
     exe = _build(tmp_path_factory, "quotient", QUOTIENT)
+    assert subprocess.run([exe]).returncode == 0
+
+
+def test_contraction_split(tmp_path_factory):
+    exe = _build(tmp_path_factory, "split", SPLIT)
     assert subprocess.run([exe]).returncode == 0
