@@ -70,13 +70,12 @@ ln_adjoint (int mode)
     return ln_mse (mode) || mode == LN_PZ_GRAD;
 }
 
-constexpr int LN_MAX_WARPS = 16;
 // dynamic shared memory that needs no attribute beside the static arrays
 constexpr size_t LN_PLAIN_SMEM = 40 * 1024;
 constexpr int LN_MAX_VPR = 10;           // voxels a region (line_plan)
 constexpr int LN_REGS = 64;             // four blocks of eight warps per SM
 constexpr int LN_WARPS = 8;             // warps a block (see line_plan)
-constexpr double LN_EDGE = 2.5;         // a block's start and end, in voxels
+constexpr double LN_EDGE = 2.5;         // a block's start and end, in voxel rows along y
 
 typedef unsigned long long u64;
 
@@ -575,11 +574,11 @@ __global__ void __maxnreg__ (LN_REGS)
 line_kernel (const __grid_constant__ LineArgs a)
 {
     extern __shared__ __align__ (16) uint8_t sm[];
-    __shared__ double sh_v[LN_MAX_WARPS];
-    __shared__ int sh_n[LN_MAX_WARPS];
+    __shared__ double sh_v[LN_WARPS];
+    __shared__ int sh_n[LN_WARPS];
     // each thread's own sums
-    __shared__ double t_v[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
-    __shared__ int t_n[ln_mse (MODE) ? 32 * LN_MAX_WARPS : 1];
+    __shared__ double t_v[ln_mse (MODE) ? 32 * LN_WARPS : 1];
+    __shared__ int t_n[ln_mse (MODE) ? 32 * LN_WARPS : 1];
     // (the contraction's blocks may start as this grid's last ones end)
     if (ln_adjoint (MODE)) asm volatile ("griddepcontrol.launch_dependents;");
     if (ln_mse (MODE)) {
@@ -1145,8 +1144,8 @@ line_plan (const BspGeom& g, LinePlan* p, int sm_count)
     }
     p->kx = std::min (g.rdims[0], 32 / g.vpr[0] + 1);
     // Tiles a block along y: an SM's share is whole blocks, and a block's
-    // start and end (its z contraction, the three extra rows) cost LN_EDGE
-    // tiles' voxels.
+    // start and end (its z contraction, the three extra rows) cost as much as
+    // LN_EDGE voxel rows.
     double best = 0.0;
     p->ty = 0;
     for (int ty = 1; ty <= g.rdims[1]; ty++) {
