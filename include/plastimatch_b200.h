@@ -185,16 +185,23 @@ int b200bsp_set_stream (b200bsp_ctx* ctx, void* stream);
 int b200bsp_score_mse (b200bsp_ctx* ctx, const float* coeff, float* score,
     float* grad, int64_t* num_vox);
 
-/* As b200bsp_score_mse with double-precision outputs (the device
- * accumulates the score and gradient in double; this skips the final
- * rounding to float). */
+/* As b200bsp_score_mse with double-precision outputs: the final rounding to
+ * float is skipped.  The score's sum is in double; so are the gradient's
+ * outer sums, over the tiles along x on the line kernel (whose sums along y
+ * and z are some tens of products each, in float) and over all tiles on the
+ * other kernels (whose sums over a tile are in float).  Its rounding, with
+ * exact positions: 3e-8 to 5e-8 (relative L2) on the line kernel, 4e-7 to
+ * 4e-6 on the tile kernel. */
 int b200bsp_score_mse_f64 (b200bsp_ctx* ctx, const float* coeff,
     double* score, double* grad, int64_t* num_vox);
 
 /* Mattes mutual information with PVI-8 histograms, flavour g semantics
  * (src/register/bspline_mi.cxx:1505-1750): score = -MI, gradient dS/dp,
  * plus the histograms of pass 1 when f_hist/m_hist/j_hist are non-NULL
- * (host pointers; bins, bins, bins*bins doubles). */
+ * (host pointers; bins, bins, bins*bins doubles).  Where the line kernel
+ * runs, it takes pass 1 and the tile kernel pass 2: their positions agree to
+ * some 1e-5 voxel, so that a voxel on the very edge of the moving image may
+ * be counted by one and not by the other. */
 int b200bsp_score_mi (b200bsp_ctx* ctx, const float* coeff, float* score,
     float* grad, int64_t* num_vox, double* f_hist, double* m_hist,
     double* j_hist);
@@ -455,7 +462,9 @@ void b200bsp_lbfgs_default_parms (b200bsp_lbfgs_parms* parms);
  * or device) holds x0 on entry; on return it holds what Plastimatch's
  * transform holds after its optimiser: the last evaluated coefficients
  * (a stop inside a line search leaves the last trial point there), and
- * res->score the last evaluated total score.  The first run on a context
+ * res->score the last evaluated total score -- of the tensor-core kernel that
+ * the optimiser keeps to, which differs from b200bsp_score's at the same
+ * coefficients by rounding where that runs the line kernel.  The first run on a context
  * allocates the optimiser's device vectors ((2m + 5) doubles and 2 floats
  * per coefficient); the context keeps them for later runs with the same m
  * and frees them with itself. */

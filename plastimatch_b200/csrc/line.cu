@@ -18,10 +18,11 @@
 // run in an order of their own: results do not depend on how blocks are
 // scheduled.
 //
-// Measured at 256x256x128, 5 voxels a region, nearest gradient: 67 us and 13
-// us for the contraction, where the tcgen05 tile kernel takes 160 and 7 us
-// (64x64x64, 8 voxels: 8 + 9 against 22 + 5 us; 512x512x160, 10x10x4: 316 +
-// 36 against 800 + 40 us).  The tensor cores' field must be carried through
+// Measured at 256x256x128, 5 voxels a region, nearest gradient: 66 us and 17
+// us for the contraction (one after the other; 82 us a call), where the
+// tcgen05 tile kernel takes 160 and 7 us (64x64x64, 8 voxels: 7 + 9, 14.4 us
+// a call, against 22 + 5 us; 512x512x160, 10x10x4: 311 + 31, 340 us a call,
+// against 800 + 40 us).  The tensor cores' field must be carried through
 // shared memory to the x order and their adjoint operand split into bf16
 // pairs, which costs more instructions than 24 two-wide multiply-adds.
 // What bounds it: 147 instructions a voxel, some 60 of them address and clamp
@@ -368,8 +369,8 @@ line_adjoint (const u64* w, u64 cxy, float cz, Row (&q)[4])
 // A voxel outside has read the moving image's border, which may hold
 // infinities or NaN, so that a derivative times 0 is not enough: its gradient
 // is the triple of zeros (line_load; one select), or its derivative is
-// selected (three: 83.9 us against 82.4 at 256x256x128 vpr 5, 30.7 against
-// 28.7 at 131x117x83 vpr 6 oblique, with spills).
+// selected (three: 83.9 us a call against 82.1 at 256x256x128 vpr 5, 30.7
+// against 26.6 at 131x117x83 vpr 6 oblique, with spills).
 template <int MODE, bool ROI, int R>
 __device__ __forceinline__ void
 line_use (const LineArgs& a, int ly, const Vox& v,

@@ -23,7 +23,7 @@ from plastimatch_b200.geometry import BsplineGrid
 pytestmark = pytest.mark.gpu
 
 # "tc-xlane": the tensor-core form with its x-lane kernel pinned (the
-# default runs MI on the tile kernel)
+# default runs PVI-8's pass 1 on the line kernel, pass 2 on the tile kernel)
 FORMS = ["fp32", "tc", "tc-xlane"]
 
 
